@@ -56,6 +56,67 @@ __device__ __forceinline__ void st_v8(void *p, const uint32_t (&w)[8]) {
 		   "r"(w[6]), "r"(w[7]) : "memory");
 }
 
+// Programmatic dependent launch (launch.h): holds the CTA until the stream's
+// previous kernel has ended and its writes are visible. Every CTA of a
+// chained kernel calls it before its first access to memory another kernel
+// may use.
+__device__ __forceinline__ void pdl_wait() {
+	asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+// Thread-block clusters: the CTA's rank, the cluster barrier in its two
+// halves, and accesses to another CTA's shared memory by element width.
+__device__ __forceinline__ uint32_t cluster_rank() {
+	uint32_t r;
+	asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+	return r;
+}
+__device__ __forceinline__ void cluster_arrive() {
+	asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+	asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t map_shared(uint32_t addr, uint32_t rank) {
+	uint32_t r;
+	asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+	return r;
+}
+template <typename T>
+__device__ __forceinline__ T ld_dsmem(uint32_t a) {
+	if constexpr (sizeof(T) == 8) {
+		uint64_t v;
+		asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(v) : "r"(a) : "memory");
+		return __builtin_bit_cast(T, v);
+	} else if constexpr (sizeof(T) == 4) {
+		uint32_t v;
+		asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+		return __builtin_bit_cast(T, v);
+	} else {
+		uint16_t v;
+		if constexpr (sizeof(T) == 2)
+			asm volatile("ld.shared::cluster.u16 %0, [%1];" : "=h"(v) : "r"(a) : "memory");
+		else
+			asm volatile("ld.shared::cluster.u8 %0, [%1];" : "=h"(v) : "r"(a) : "memory");
+		if constexpr (sizeof(T) == 2) return __builtin_bit_cast(T, v);
+		else return __builtin_bit_cast(T, (uint8_t)v);
+	}
+}
+template <typename T>
+__device__ __forceinline__ void st_dsmem(uint32_t a, T x) {
+	if constexpr (sizeof(T) == 8)
+		asm volatile("st.shared::cluster.u64 [%0], %1;"
+			:: "r"(a), "l"(__builtin_bit_cast(uint64_t, x)) : "memory");
+	else if constexpr (sizeof(T) == 4)
+		asm volatile("st.shared::cluster.u32 [%0], %1;"
+			:: "r"(a), "r"(__builtin_bit_cast(uint32_t, x)) : "memory");
+	else if constexpr (sizeof(T) == 2)
+		asm volatile("st.shared::cluster.u16 [%0], %1;"
+			:: "r"(a), "h"(__builtin_bit_cast(uint16_t, x)) : "memory");
+	else
+		asm volatile("st.shared::cluster.u8 [%0], %1;"
+			:: "r"(a), "h"((uint16_t)__builtin_bit_cast(uint8_t, x)) : "memory");
+}
+
 // Spin budget of every bounded wait: with the nanosleep back-off below and
 // the re-read of the flag each round this is about a second of waiting
 // before a wait gives up.

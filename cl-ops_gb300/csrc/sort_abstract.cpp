@@ -352,7 +352,7 @@ struct AbitonicData {
 const char *sbitonic_init(CloSort *s, const char *options, GError **err) {
 	(void)options;
 	s->data = nullptr;
-	return "sm_103a:sbitonic(one network step per launch)";
+	return "sm_103a:sbitonic(shared-memory tiles + register passes)";
 }
 
 const char *abitonic_init(CloSort *s, const char *options, GError **err) {
@@ -404,40 +404,28 @@ void bitonic_finalize(CloSort *s) {
 	s->data = nullptr;
 }
 
-}  // namespace
-
-namespace clo {
-// Implemented in bitonic.cu: one global compare-exchange step per launch,
-// and the grouped form with explicit grouping limits.
-cudaError_t bitonic_sort_simple(void *data, size_t n, CloType type,
-	CCLContext *ctx, cudaStream_t s, GError **err);
-cudaError_t bitonic_sort_tuned(void *data, size_t n, CloType type, int max_ps,
-	int max_sfs, CCLContext *ctx, cudaStream_t s, GError **err);
-}
-
-namespace {
-
 CCLEvent *bitonic_sort_common(CloSort *s, CCLQueue *q, CCLBuffer *in,
 	CCLBuffer *out, size_t numel, bool simple, GError **err) {
 	if (!check_numel(s, in, numel, err)) return nullptr;
 	ccl_event *ev = clo::event_begin(q, simple ? "sbitonic" : "abitonic");
-	CCLBuffer *tgt = target_buffer(s, q, in, out, numel, err);
-	if (!tgt) return nullptr;
-	// abitonic's maxps bounds the steps grouped per global pass and maxsfs
-	// the largest step finished in shared memory (clo_sort_abitonic.c:
-	// 155-157); neither changes the result.
 	if (s->jit) {
+		CCLBuffer *tgt = target_buffer(s, q, in, out, numel, err);
+		if (!tgt) return nullptr;
 		if (!jit_sort(s, q, tgt->ptr, tgt->ptr, numel, JIT_BITONIC, err)) return nullptr;
 		clo::event_end(ev);
 		return ev;
 	}
+	if (out == nullptr) out = in;
+	if (out != in && !check_numel(s, out, numel, err)) return nullptr;
+	// abitonic's maxps bounds the steps grouped per global pass and maxsfs
+	// the largest step finished in shared memory (clo_sort_abitonic.c:
+	// 155-157); neither changes the result. sbitonic has no settings: its
+	// steps are grouped like abitonic's (one launch per step, the reference's
+	// form, took 0.56 ms for 2^16 keys).
 	AbitonicData *d = (AbitonicData *)s->data;
-	cudaError_t e = simple
-		? clo::bitonic_sort_simple(tgt->ptr, numel, s->elem_type, s->ctx,
-			q->stream, err)
-		: clo::bitonic_sort_tuned(tgt->ptr, numel, s->elem_type,
-			d ? (int)d->max_ps : 4,
-			d && d->max_sfs < 64 ? (int)d->max_sfs : 0, s->ctx, q->stream, err);
+	cudaError_t e = clo::bitonic_sort(in->ptr, out->ptr, numel, s->elem_type,
+		d ? (int)d->max_ps : 4, d && d->max_sfs < 64 ? (int)d->max_sfs : 0, s->ctx, q->stream,
+		err);
 	if (e != cudaSuccess) return nullptr;
 	clo::event_end(ev);
 	return ev;
