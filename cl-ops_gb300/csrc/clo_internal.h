@@ -119,14 +119,13 @@ bool type_is_signed(CloType t);
 // Kernel launchers (implemented in *.cu).
 // ---------------------------------------------------------------------
 
-// Stable LSD radix sort (onesweep) of n keys of key_bytes in {1,2,4,8},
-// ascending by bits [0, sort_bits) of the unsigned key pattern, carrying
-// optional values of val_bytes in {0,4,8}. In place on keys/vals.
-// `allow_skip` lets the launcher read back the digit histograms and skip
-// passes whose digit is constant (not allowed during graph capture).
-cudaError_t radix_sort(void *keys, void *vals, size_t n, int key_bytes,
-	int val_bytes, int sort_bits, CCLContext *ctx, cudaStream_t s,
-	bool allow_skip, GError **err);
+// Stable LSD radix sort (onesweep) of n keys of key_bytes in {1,2,4,8} from
+// src into dst (which may be src), ascending by bits [0, sort_bits) of the
+// unsigned key pattern, carrying optional values of val_bytes in {0,4,8},
+// which are sorted in place. Passes whose digit is constant are skipped on
+// the device; nothing is read back.
+cudaError_t radix_sort(const void *src, void *dst, void *vals, size_t n, int key_bytes,
+	int val_bytes, int sort_bits, CCLContext *ctx, cudaStream_t s, GError **err);
 
 // Stable partition of n keys (key_bytes 2, 4 or 8) by the top 8 bits of
 // their low sort_bits bits, into keys_out; counts (host, 256 entries)

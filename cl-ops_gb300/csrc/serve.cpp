@@ -185,16 +185,12 @@ void launch_batch(clo_server *srv, Batch *b, Lane *lane) {
 			clo::tmp_free(dev, s);
 		}
 	} else if (dev_data && k == 1) {
-		// One device-resident request: the plain kernels on its buffers
-		// (a sort copies its input to the output and sorts there).
+		// One device-resident request: the plain kernels on its buffers.
 		const size_t ib = elem_bytes(r0.type);
 		const size_t ob = r0.op == CLO_SERVE_SCAN ? elem_bytes(r0.sum_type) : ib;
 		if (r0.n && r0.op == CLO_SERVE_SORT) {
-			if (r0.out != r0.in)
-				e = cudaMemcpyAsync(r0.out, r0.in, r0.n * ib, cudaMemcpyDeviceToDevice, s);
-			if (e == cudaSuccess)
-				e = clo::radix_sort(r0.out, nullptr, r0.n, (int)ib, 0, (int)(8 * ib), srv->ctx,
-					s, false, &err);
+			e = clo::radix_sort(r0.in, r0.out, nullptr, r0.n, (int)ib, 0, (int)(8 * ib),
+				srv->ctx, s, &err);
 		} else if (r0.n) {
 			e = clo::scan_exclusive(r0.in, r0.out, r0.n, r0.type, (int)ob, srv->ctx, s, &err);
 		}
@@ -238,12 +234,11 @@ void launch_batch(clo_server *srv, Batch *b, Lane *lane) {
 				}
 			}
 			if (e == cudaSuccess && total > 0) {
-				// A request alone takes the plain kernels (the onesweep
-				// sort, without the host readback of pass skipping);
-				// a batch takes one segmented call.
+				// A request alone takes the plain kernels; a batch takes one
+				// segmented call.
 				if (r0.op == CLO_SERVE_SORT && k == 1)
-					e = clo::radix_sort(din, nullptr, total, (int)ib, 0, (int)(8 * ib),
-						srv->ctx, s, false, &err);
+					e = clo::radix_sort(din, din, nullptr, total, (int)ib, 0, (int)(8 * ib),
+						srv->ctx, s, &err);
 				else if (r0.op == CLO_SERVE_SORT)
 					e = clo::seg_sort(din, total, d_off, k, (int)ib, (int)(8 * ib), 0,
 						srv->ctx, s, &err);

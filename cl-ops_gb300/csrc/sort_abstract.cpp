@@ -160,8 +160,8 @@ bool jit_sort(CloSort *s, CCLQueue *q, void *src, void *dst, size_t numel,
 		void *a1[] = {&src, &keys, &idx, &n};
 		bool ok = cuda_ok(clo::jit_launch(j.keys, numel, a1, st, sms), err, "get_key");
 		const int bits = (int)(8 * (eb < kb ? eb : kb));
-		ok = ok && clo::radix_sort(keys, idx, numel, (int)kb, 4, bits, s->ctx, st,
-			!clo::stream_capturing(st), err) == cudaSuccess;
+		ok = ok && clo::radix_sort(keys, keys, idx, numel, (int)kb, 4, bits, s->ctx, st, err) ==
+			cudaSuccess;
 		void *a2[] = {&src, &idx, &sorted, &n};
 		ok = ok && cuda_ok(clo::jit_launch(j.gather, numel, a2, st, sms), err, "gather");
 		ok = ok && cuda_ok(cudaMemcpyAsync(dst, sorted, numel * eb,
@@ -298,17 +298,18 @@ CCLEvent *satradix_sort(CloSort *s, CCLQueue *cq_exec, CCLQueue *cq_comm,
 		return nullptr;
 	}
 	ccl_event *ev = clo::event_begin(cq_exec, "satradix");
-	CCLBuffer *tgt = target_buffer(s, cq_exec, in, out, numel, err);
-	if (!tgt) return nullptr;
 	if (s->jit) {
+		CCLBuffer *tgt = target_buffer(s, cq_exec, in, out, numel, err);
+		if (!tgt) return nullptr;
 		if (!jit_sort(s, cq_exec, tgt->ptr, tgt->ptr, numel, JIT_RADIX, err)) return nullptr;
 		clo::event_end(ev);
 		return ev;
 	}
+	if (out == nullptr) out = in;
+	if (out != in && !check_numel(s, out, numel, err)) return nullptr;
 	int kb = (int)clo_type_sizeof(s->elem_type);
-	bool skip = !clo::stream_capturing(cq_exec->stream);
-	if (clo::radix_sort(tgt->ptr, nullptr, numel, kb, 0, satradix_sort_bits(s),
-			s->ctx, cq_exec->stream, skip, err) != cudaSuccess)
+	if (clo::radix_sort(in->ptr, out->ptr, nullptr, numel, kb, 0, satradix_sort_bits(s),
+			s->ctx, cq_exec->stream, err) != cudaSuccess)
 		return nullptr;
 	clo::event_end(ev);
 	return ev;
@@ -889,10 +890,8 @@ CCLEvent *clo_sort_kv_with_device_data(CloSort *sorter, CCLQueue *q,
 	ccl_event *ev = clo::event_begin(q, radix ? "satradix_kv" : "gselect_kv");
 	size_t kb = clo_type_sizeof(sorter->elem_type);
 	if (radix) {
-		bool skip = !clo::stream_capturing(q->stream);
-		if (clo::radix_sort(keys->ptr, values->ptr, numel, (int)kb, (int)vb,
-				satradix_sort_bits(sorter), sorter->ctx, q->stream, skip,
-				err) != cudaSuccess)
+		if (clo::radix_sort(keys->ptr, keys->ptr, values->ptr, numel, (int)kb, (int)vb,
+				satradix_sort_bits(sorter), sorter->ctx, q->stream, err) != cudaSuccess)
 			return nullptr;
 	} else {
 		void *tk = clo::tmp_alloc(sorter->ctx, numel * kb, q->stream, err);
