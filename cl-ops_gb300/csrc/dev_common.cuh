@@ -56,6 +56,18 @@ __device__ __forceinline__ void st_v8(void *p, const uint32_t (&w)[8]) {
 		   "r"(w[6]), "r"(w[7]) : "memory");
 }
 
+// The same, streaming (evict-first).
+__device__ __forceinline__ void ld_stream_v8(const void *p, uint32_t (&w)[8]) {
+	asm volatile("ld.global.cs.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+		: "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]),
+		  "=r"(w[6]), "=r"(w[7]) : "l"(p));
+}
+__device__ __forceinline__ void st_stream_v8(void *p, const uint32_t (&w)[8]) {
+	asm volatile("st.global.cs.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+		:: "l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]),
+		   "r"(w[6]), "r"(w[7]) : "memory");
+}
+
 // Programmatic dependent launch (launch.h): holds the CTA until the stream's
 // previous kernel has ended and its writes are visible. Every CTA of a
 // chained kernel calls it before its first access to memory another kernel

@@ -7,40 +7,34 @@
 // Integer addition is associative, so the result is bit-identical to the
 // reference's work-group Blelloch trees whatever the summation order.
 //
-// Layout: tiles of 8192 elements, 256 threads. Each warp owns 1024
-// consecutive elements as two blocks of 512, lane l holding elements
-// 16 l .. 16 l + 15 of each block. A block moves between global memory and
-// shared memory with coalesced 16-byte vector accesses through a padded
-// transpose (conflict-free per-lane runs). Inputs stay in shared memory:
-// the thread and warp sums are taken before the lookback and the outputs
-// are formed by a second read after it, so no per-element state is held
-// in registers across the wait. Tiles take ids from an atomic counter (so
-// a tile only ever waits on tiles already running), publish their
-// aggregate, then warp 0 looks back over a 64-tile window per round trip
-// until it meets an inclusive prefix. Status words carry their own ready
-// bits, so neither side needs a memory fence. Every wait is bounded.
-//
-// The lookback bounds the rate of tiles, not of bytes: a window of 64
-// tiles per L2 round trip, so the tile is made large enough (8192
-// elements, 96 KB of uint -> ulong traffic) that the tile rate HBM needs
-// stays well inside it.
+// Layout (scan_rows.cuh): tiles of 8192 elements, 256 threads, held in
+// registers as rows of whole vectors per lane; a row's scan is a warp scan of
+// the lanes' run sums. Tiles take ids from an atomic counter (so a tile only
+// ever waits on tiles already running), publish their aggregate, then warp 0
+// looks back over a 64-tile window per round trip until it meets an
+// inclusive prefix. Status words carry their own ready bits, so neither side
+// needs a memory fence. Every wait is bounded. Staging the tile in shared
+// memory (a lane scanning 16 consecutive elements, seven shared wavefronts
+// per 32 elements for uint -> ulong) took 589 us at 2^28 against 551.
 //
 // HBM roofline: sizeof(in) + sizeof(out) bytes per element (12 B for
-// uint -> ulong), plus 32 B of tile status per 8192 elements.
+// uint -> ulong), plus 32 B of tile status per tile.
+#include <algorithm>
 #include <atomic>
 #include <mutex>
 #include <type_traits>
 
 #include "clo_internal.h"
 #include "dev_common.cuh"
+#include "launch.h"
+#include "scan_rows.cuh"
 #include "scan_status.cuh"
-#include "scan_tile.cuh"
 #include "timing.h"
 
 namespace clo {
 namespace {
 
-using namespace scantile;
+using scanrows::Rows;
 
 using lb::Slots;
 using lb::TileStatus;
@@ -60,18 +54,53 @@ __device__ __forceinline__ Acc shfl_up(Acc v, int d) {
 // iteration) into registers and sums them, so the next tile's aggregate is
 // published as soon as the lookback ends -- before this tile's outputs are
 // written -- and no later tile waits on it longer than on a freshly
-// launched one; after the outputs the prefetched data is transposed into
-// shared memory. Every wait is on a lower tile id (down to tile 0, which
+// launched one; after the outputs the prefetched tile becomes the current
+// one. Every wait is on a lower tile id (down to tile 0, which
 // publishes its prefix at once), so the waits cannot form a cycle.
+template <typename InT, typename OutT, int THREADS, int TILE, int MINB>
+struct ScanCfg {
+	static constexpr int kThreads = THREADS, kTile = TILE, kMinBlocks = MINB;
+	using R = Rows<InT, OutT, THREADS, TILE>;
+};
+// Sums of one or two bytes, or narrower than the input: one shape for all.
 template <typename InT, typename OutT>
-__global__ void __launch_bounds__(kThreads, (scan_min_blocks<InT, OutT>()))
-scan_lookback(const InT *__restrict__ in, OutT *__restrict__ out, size_t n,
-	TileStatus ts,
-	int *dev_status, bool vec_ok, long long debug_skip_tile,
+constexpr bool kOneShape = sizeof(OutT) <= 2 || (sizeof(InT) > sizeof(OutT));
+template <bool C, typename A, typename B>
+using If = typename std::conditional<C, A, B>::type;
+
+// Threads, tile and resident CTAs per SM (registers: 65536 / (CTAs x
+// threads); the current and the prefetched tile take most of them). The tile
+// rate is bounded by the lookback (a window of 64 tiles a round trip, about
+// 80 tiles a microsecond), so narrow types take tiles twice as long. Measured
+// at 2^28 (us, 8192-element tiles at the same registers / these): uint ->
+// uint 406 / 375, uchar -> uint 404 / 255. uint -> ulong: 8192 551, 16384 at
+// one CTA 590, 512 threads 592. Windows of 96 and 128 tiles: 600 and 634.
+template <typename InT, typename OutT>
+using ScanBig = If<kOneShape<InT, OutT>, ScanCfg<InT, OutT, 256, 8192, 1>,
+	If<sizeof(OutT) == 8, ScanCfg<InT, OutT, 256, 8192, 2>,
+	If<sizeof(InT) == 4, ScanCfg<InT, OutT, 256, 16384, 2>, ScanCfg<InT, OutT, 256, 16384, 3>>>>;
+// Up to kSmallMax elements, 4096-element tiles: twice the CTAs, each with
+// half the rows to scan (2^18 uint -> ulong 6.3 us against 8.0, 2^20 8.3
+// against 9.1; 2^22 20.8 against 17.5).
+constexpr size_t kSmallMax = (size_t)1 << 20;
+template <typename InT, typename OutT>
+using ScanSmall = If<kOneShape<InT, OutT>, ScanBig<InT, OutT>,
+	If<sizeof(InT) == 8, ScanCfg<InT, OutT, 512, 4096, 2>, ScanCfg<InT, OutT, 256, 4096, 4>>>;
+// One tile of 1024 threads, in one launch without statuses (5003 uint ->
+// ulong: 8.8 us with a memset and a 256-thread tile, 3.9 so).
+template <typename InT, typename OutT>
+using ScanOne = If<kOneShape<InT, OutT>, ScanBig<InT, OutT>, ScanCfg<InT, OutT, 1024, 8192, 1>>;
+
+template <typename InT, typename OutT, typename CFG>
+__global__ void __launch_bounds__(CFG::kThreads, CFG::kMinBlocks)
+scan_lookback(const InT *in, OutT *out, size_t n, TileStatus ts,
+	int *dev_status, int vec, long long debug_skip_tile,
 	const void *carry_in, void *carry_out) {
 	using Acc = typename std::conditional<(sizeof(OutT) <= 4), uint32_t,
 		uint64_t>::type;
-	extern __shared__ __align__(16) unsigned char s_dyn[];
+	using R = typename CFG::R;
+	constexpr int kTile = R::kTile;
+	constexpr int kWarps = R::kWarps, kE = R::kE, kRows = R::kRows;
 	__shared__ Acc s_warp_tot[kWarps];
 	__shared__ Acc s_next_tot[kWarps];
 	__shared__ Acc s_excl;
@@ -79,67 +108,61 @@ scan_lookback(const InT *__restrict__ in, OutT *__restrict__ out, size_t n,
 
 	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 	const uint32_t num_tiles = (uint32_t)((n + kTile - 1) / kTile);
-	InT *s_in = reinterpret_cast<InT *>(s_dyn + (size_t)warp *
-		(kBlocks * padded<InT>() * sizeof(InT) + padded<OutT>() * sizeof(OutT)));
-	OutT *s_out = reinterpret_cast<OutT *>(s_in + kBlocks * padded<InT>());
-	auto full_tile = [&](uint32_t t) {
-		return vec_ok && (size_t)(t + 1) * kTile <= n;
+	const bool solo = num_tiles == 1;  // one tile: no statuses, no counter
+	const bool in_wide = vec & 2, out_wide = vec & 4;
+	auto full_tile = [&](uint32_t t) { return (vec & 1) && (size_t)(t + 1) * kTile <= n; };
+	// A warp's elements of a partial tile may still be whole.
+	auto full_seg = [&](size_t seg) { return (vec & 1) && seg + R::kWarpElems <= n; };
+	auto load_seg = [&](R &r, size_t seg) {
+		if (full_seg(seg)) r.load(in + seg, lane, in_wide);
+		else r.load_some(in + (seg < n ? seg : 0), lane, seg < n ? n - seg : 0);
 	};
-	if (tid == 0) s_tile = atomicAdd(ts.counter, 1u);
+	auto seg_of = [&](uint32_t t) { return (size_t)t * kTile + (size_t)warp * R::kWarpElems; };
+	dev::pdl_wait();
+	if (tid == 0) s_tile = solo ? 0u : atomicAdd(ts.counter, 1u);
 	__syncthreads();
 	uint32_t tile = s_tile;
 	if (tile >= num_tiles) return;
-	{
-		const size_t wseg = (size_t)tile * kTile + (size_t)warp * kWarpElems;
-		if (full_tile(tile)) {
-			BlockRegs<InT> r;
-			issue_loads<InT>(r, in, wseg, lane);
-			store_loads<InT>(r, s_in, lane);
-		} else {
-#pragma unroll
-			for (int b = 0; b < kBlocks; ++b)
-				load_block_scalar<InT>(in, n, wseg + (size_t)b * kBlock, s_in + b * padded<InT>(), lane);
-		}
-	}
-	__syncwarp();
+	R cur;
+	load_seg(cur, seg_of(tile));
 	bool agg_published = false;  // the current tile's aggregate is out
 
 	for (;;) {
-		if (tid == 0) s_next = atomicAdd(ts.counter, 1u);
-		const size_t wseg = (size_t)tile * kTile + (size_t)warp * kWarpElems;
+		if (tid == 0) s_next = solo ? 1u : atomicAdd(ts.counter, 1u);
 
-		// ---- lane run sums and their warp scans, per block --------------
-		Acc lane_excl[kBlocks], block_tot[kBlocks];
+		// ---- run sums, row scans, the warp's total ----------------------
+		Acc ex[kRows], inc[kRows];
 #pragma unroll
-		for (int b = 0; b < kBlocks; ++b) {
-			const InT *sin = s_in + b * padded<InT>();
+		for (int r = 0; r < kRows; ++r) {
 			Acc run = 0;
 #pragma unroll
-			for (int j = 0; j < kItems; ++j) run += (Acc)(OutT)sin[pidx<InT>(lane * kItems + j)];
-			Acc inc = run;
+			for (int e = 0; e < kE; ++e) run += (Acc)(OutT)cur.at(r, e);
+			ex[r] = run;
+			inc[r] = run;
+		}
 #pragma unroll
-			for (int d = 1; d < 32; d <<= 1) {
-				Acc t = shfl_up(inc, d);
-				if (lane >= d) inc += t;
+		for (int d = 1; d < 32; d <<= 1) {
+#pragma unroll
+			for (int r = 0; r < kRows; ++r) {
+				const Acc t = shfl_up(inc[r], d);
+				if (lane >= d) inc[r] += t;
 			}
-			lane_excl[b] = inc - run;
-			block_tot[b] = __shfl_sync(0xffffffffu, inc, 31);
 		}
-		if (lane == 0) {
-			Acc wsum = 0;
+		Acc wsum = 0;
 #pragma unroll
-			for (int b = 0; b < kBlocks; ++b) wsum += block_tot[b];
-			s_warp_tot[warp] = wsum;
+		for (int r = 0; r < kRows; ++r) {
+			ex[r] = inc[r] - ex[r] + wsum;
+			wsum += __shfl_sync(0xffffffffu, inc[r], 31);
 		}
+		if (lane == 0) s_warp_tot[warp] = wsum;
 		__syncthreads();
 		const uint32_t next = s_next;
 		const bool have_next = next < num_tiles;
 		const bool next_full = have_next && full_tile(next);
-		const size_t nseg = (size_t)next * kTile + (size_t)warp * kWarpElems;
 
 		// ---- prefetch of the next tile (all warps) ----------------------
-		BlockRegs<InT> r;
-		if (next_full) issue_loads<InT>(r, in, nseg, lane);
+		R nxt;
+		if (next_full) nxt.load(in + seg_of(next), lane, in_wide);
 		const bool next_publish = next_full && (long long)next != debug_skip_tile;
 
 		// ---- tile aggregate, publication and lookback (warp 0) ----------
@@ -153,7 +176,7 @@ scan_lookback(const InT *__restrict__ in, OutT *__restrict__ out, size_t n,
 			}
 			const Acc aggregate = __shfl_sync(0xffffffffu, winc, kWarps - 1);
 			if (lane < kWarps) s_warp_tot[lane] = winc - wt;  // warp exclusive
-			const bool do_publish = (long long)tile != debug_skip_tile;
+			const bool do_publish = (long long)tile != debug_skip_tile && !solo;
 			constexpr int PT = Slots<Acc>::kPerTile;
 			Acc excl = 0;
 			if (tile == 0) {
@@ -177,16 +200,11 @@ scan_lookback(const InT *__restrict__ in, OutT *__restrict__ out, size_t n,
 		}
 		// The next tile's sum from the prefetched registers.
 		if (next_full) {
-			constexpr int EPC = BlockRegs<InT>::kEpc;
 			Acc part = 0;
 #pragma unroll
-			for (int b = 0; b < kBlocks; ++b)
+			for (int r = 0; r < kRows; ++r)
 #pragma unroll
-				for (int k = 0; k < BlockRegs<InT>::kPerLane; ++k) {
-					const InT *e = reinterpret_cast<const InT *>(&r.v[b][k]);
-#pragma unroll
-					for (int q = 0; q < EPC; ++q) part += (Acc)(OutT)e[q];
-				}
+				for (int e = 0; e < kE; ++e) part += (Acc)(OutT)nxt.at(r, e);
 			part = warp_sum<Acc>(part);
 			if (lane == 0) s_next_tot[warp] = part;
 		}
@@ -198,61 +216,54 @@ scan_lookback(const InT *__restrict__ in, OutT *__restrict__ out, size_t n,
 			publish<Acc>(ts.words + (size_t)next * Slots<Acc>::kPerTile, agg);
 		}
 
-		// ---- outputs per block: second read, staged, coalesced stores ----
-		Acc base = s_excl + s_warp_tot[warp];
+		// ---- outputs, straight from the registers ------------------------
+		const Acc base = s_excl + s_warp_tot[warp];
+		const size_t seg = seg_of(tile);
+		const bool full = full_seg(seg);
 #pragma unroll
-		for (int b = 0; b < kBlocks; ++b) {
-			const InT *sin = s_in + b * padded<InT>();
-			Acc run = base + lane_excl[b];
+		for (int r = 0; r < kRows; ++r) {
+			Acc run = base + ex[r];
+			const size_t i0 = seg + (size_t)(32 * r + lane) * kE;
+			if (full) {
+				uint32_t o[8];
 #pragma unroll
-			for (int j = 0; j < kItems; ++j) {
-				const int q = lane * kItems + j;
-				const Acc v = (Acc)(OutT)sin[pidx<InT>(q)];
-				s_out[pidx<OutT>(q)] = (OutT)run;
-				run += v;
-			}
-			base += block_tot[b];
-			__syncwarp();
-			const size_t seg = wseg + (size_t)b * kBlock;
-			if (seg + kBlock <= n && vec_ok) {
-				constexpr int EPC = 16 / sizeof(OutT);
-				constexpr int CHUNKS = kBlock / EPC;
-				uint4 *dst = reinterpret_cast<uint4 *>(out + seg);
-#pragma unroll
-				for (int c = lane; c < CHUNKS; c += 32) {
-					uint4 v;
-					OutT *e = reinterpret_cast<OutT *>(&v);
-#pragma unroll
-					for (int k = 0; k < EPC; ++k) e[k] = s_out[pidx<OutT>(c * EPC + k)];
-					dev::st_stream_v4(dst + c, v);
+				for (int e = 0; e < kE; ++e) {
+					scanrows::pack<OutT>(o, e, (OutT)run);
+					run += (Acc)(OutT)cur.at(r, e);
 				}
+				scanrows::store_run(out + i0, o, out_wide);
 			} else {
-				for (int i = lane; i < kBlock; i += 32)
-					if (seg + i < n) out[seg + i] = s_out[pidx<OutT>(i)];
+#pragma unroll
+				for (int e = 0; e < kE; ++e) {
+					if (i0 + e < n) out[i0 + e] = (OutT)run;
+					run += (Acc)(OutT)cur.at(r, e);
+				}
 			}
-			__syncwarp();
 		}
 		if (!have_next) break;
 
-		// ---- the next tile into shared memory ---------------------------
+		// ---- on to the next tile ------------------------------------------
 		if (next_full) {
-			store_loads<InT>(r, s_in, lane);
+			cur = nxt;
 		} else {
-#pragma unroll
-			for (int b = 0; b < kBlocks; ++b)
-				load_block_scalar<InT>(in, n, nseg + (size_t)b * kBlock, s_in + b * padded<InT>(), lane);
+			load_seg(cur, seg_of(next));
 		}
-		__syncwarp();
 		agg_published = next_full;
 		tile = next;
 	}
 }
 
-// Per device and type pair, once: opts the kernel into its dynamic shared
-// memory (more than 48 KB for most pairs) and records its resident CTAs
-// per SM. Later calls (possibly while a graph is being captured) only read
+// Clears the tile statuses and the counter.
+__global__ void __launch_bounds__(256) scan_prep(uint4 *words, size_t count) {
+	dev::pdl_wait();
+	for (size_t i = blockIdx.x * (size_t)256 + threadIdx.x; i < count; i += (size_t)gridDim.x * 256)
+		words[i] = make_uint4(0, 0, 0, 0);
+}
+
+// Per device and type pair, once: records the kernel's resident CTAs per SM.
+// Later calls (possibly while a graph is being captured) only read
 // the cached count.
-template <typename InT, typename OutT>
+template <typename InT, typename OutT, typename CFG>
 cudaError_t scan_prepare(int *per_sm) {
 	static std::atomic<int> cached[64];
 	static std::mutex mu;
@@ -265,11 +276,8 @@ cudaError_t scan_prepare(int *per_sm) {
 		std::lock_guard<std::mutex> lk(mu);
 		v = cached[dev].load(std::memory_order_relaxed);
 		if (v == 0) {
-			e = cudaFuncSetAttribute(scan_lookback<InT, OutT>,
-				cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scan_smem<InT, OutT>());
-			if (e == cudaSuccess)
-				e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, scan_lookback<InT, OutT>,
-					kThreads, scan_smem<InT, OutT>());
+			e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, scan_lookback<InT, OutT, CFG>,
+				CFG::kThreads, 0);
 			if (e != cudaSuccess) return e;
 			if (v < 1) v = 1;
 			cached[dev].store(v, std::memory_order_release);
@@ -285,41 +293,65 @@ inline unsigned scan_grid(size_t tiles, int per_sm, int sm_count) {
 	return (unsigned)std::max<size_t>(g, 1);
 }
 
-template <typename InT, typename OutT>
-cudaError_t launch_scan(const void *in, void *out, size_t n, CCLContext *ctx,
+// The kernel's vector flags: 1 both arrays 16-byte aligned, 2 and 4 the input
+// and the output 32-byte aligned.
+inline int scan_vec(const void *in, const void *out) {
+	const uintptr_t a = (uintptr_t)in, b = (uintptr_t)out;
+	return ((a | b) % 16 == 0 ? 1 : 0) | (a % 32 == 0 ? 2 : 0) | (b % 32 == 0 ? 4 : 0);
+}
+
+template <typename InT, typename OutT, typename CFG>
+cudaError_t launch_scan_cfg(const void *in, void *out, size_t n, CCLContext *ctx,
 	cudaStream_t s, GError **err, long long debug_skip_tile,
 	const void *carry_in = nullptr, void *carry_out = nullptr) {
 	using Acc = typename std::conditional<(sizeof(OutT) <= 4), uint32_t,
 		uint64_t>::type;
-	const size_t tiles = (n + kTile - 1) / kTile;
+	const size_t tiles = (n + CFG::kTile - 1) / CFG::kTile;
 	if (tiles >= (1ull << 31)) {
 		set_error(err, CLO_ERROR_ARGS, "Scan of %zu elements is too large", n);
 		return cudaErrorInvalidValue;
 	}
+	// One tile needs no statuses.
 	const size_t status_bytes = tiles * Slots<Acc>::kPerTile * sizeof(uint64_t);
 	const size_t bytes = status_bytes + 16;
-	char *tmp = (char *)tmp_alloc(ctx, bytes, s, err);
-	if (!tmp) return cudaErrorMemoryAllocation;
-	TileStatus ts;
-	ts.words = (uint64_t *)tmp;
-	ts.counter = (uint32_t *)(tmp + status_bytes);
-	cudaError_t e = cudaMemsetAsync(tmp, 0, bytes, s);
-	bool vec_ok = ((uintptr_t)in % 16 == 0) && ((uintptr_t)out % 16 == 0);
+	char *tmp = nullptr;
+	TileStatus ts = {nullptr, nullptr};
+	cudaError_t e = cudaSuccess;
+	if (tiles > 1) {
+		tmp = (char *)tmp_alloc(ctx, bytes, s, err);
+		if (!tmp) return cudaErrorMemoryAllocation;
+		ts.words = (uint64_t *)tmp;
+		ts.counter = (uint32_t *)(tmp + status_bytes);
+		const size_t vecs = bytes / 16;
+		e = launch_chained(scan_prep, (unsigned)std::min<size_t>((vecs + 1023) / 1024, 64), 256, 0,
+			s, 1, (uint4 *)tmp, vecs);
+		count_launches(1);
+	}
 	int per_sm = 1;
-	if (e == cudaSuccess) e = scan_prepare<InT, OutT>(&per_sm);
+	if (e == cudaSuccess) e = scan_prepare<InT, OutT, CFG>(&per_sm);
 	if (e == cudaSuccess) {
 		KernelTimer t("scan_lookback", s, (double)n * (sizeof(InT) + sizeof(OutT)));
-		scan_lookback<InT, OutT><<<scan_grid(tiles, per_sm, ctx->sm_count), kThreads,
-			scan_smem<InT, OutT>(), s>>>(
-			(const InT *)in, (OutT *)out, n, ts, ctx->d_status, vec_ok,
-			debug_skip_tile, carry_in, carry_out);
+		e = launch_chained(scan_lookback<InT, OutT, CFG>, scan_grid(tiles, per_sm, ctx->sm_count),
+			CFG::kThreads, 0, s, 1, (const InT *)in, (OutT *)out, n, ts, ctx->d_status,
+			scan_vec(in, out), debug_skip_tile, carry_in, carry_out);
 		t.stop();
 		count_launches(1);
-		e = cudaGetLastError();
 	}
 	tmp_free(tmp, s);
 	if (e != cudaSuccess) cuda_ok(e, err, "scan_lookback");
 	return e;
+}
+
+template <typename InT, typename OutT>
+cudaError_t launch_scan(const void *in, void *out, size_t n, CCLContext *ctx,
+	cudaStream_t s, GError **err, long long debug_skip_tile, const void *ci, void *co) {
+	auto go = [&](auto cfg) {
+		return launch_scan_cfg<InT, OutT, decltype(cfg)>(in, out, n, ctx, s, err, debug_skip_tile, ci,
+			co);
+	};
+	if (n <= ScanOne<InT, OutT>::kTile) return go(ScanOne<InT, OutT>());
+	if (n <= kSmallMax) return go(ScanSmall<InT, OutT>());
+	return go(ScanBig<InT, OutT>());
 }
 
 template <typename InT>
@@ -390,7 +422,8 @@ extern "C" void clo_gb300_debug_scan_withhold(long long tile) {
 // cudaGetSymbolAddress and cached.
 // ---------------------------------------------------------------------
 
-// Largest no-allocation scan: 2^15 tiles of 8192 elements = 2^28 elements.
+// Largest no-allocation scan: 2^15 tiles of 8192 elements (the smallest its
+// shapes take) = 2^28 elements.
 #define CLO_NOALLOC_MAX_TILES (1u << 15)
 // Four status words per tile (64-bit sums) and one word for the counter.
 #define CLO_NOALLOC_WORDS (CLO_NOALLOC_MAX_TILES * 4u + 2u)
@@ -400,7 +433,7 @@ static __device__ __align__(256) uint64_t g_scan_noalloc_scratch[CLO_NOALLOC_WOR
 namespace clo {
 namespace {
 
-constexpr size_t kNoAllocMaxElems = (size_t)CLO_NOALLOC_MAX_TILES * kTile;
+constexpr size_t kNoAllocMaxElems = (size_t)CLO_NOALLOC_MAX_TILES * 8192;
 static_assert(kNoAllocMaxElems == ((size_t)1 << 28), "no-allocation scan limit");
 
 std::mutex g_noalloc_mu;
@@ -426,10 +459,10 @@ struct CurrentDevice {
 template <typename InT>
 cudaError_t noalloc_prepare_in() {
 	int v = 0;
-	cudaError_t e = scan_prepare<InT, uint8_t>(&v);
-	if (e == cudaSuccess) e = scan_prepare<InT, uint16_t>(&v);
-	if (e == cudaSuccess) e = scan_prepare<InT, uint32_t>(&v);
-	if (e == cudaSuccess) e = scan_prepare<InT, uint64_t>(&v);
+	cudaError_t e = scan_prepare<InT, uint8_t, ScanBig<InT, uint8_t>>(&v);
+	if (e == cudaSuccess) e = scan_prepare<InT, uint16_t, ScanBig<InT, uint16_t>>(&v);
+	if (e == cudaSuccess) e = scan_prepare<InT, uint32_t, ScanBig<InT, uint32_t>>(&v);
+	if (e == cudaSuccess) e = scan_prepare<InT, uint64_t, ScanBig<InT, uint64_t>>(&v);
 	return e;
 }
 
@@ -478,7 +511,8 @@ cudaError_t launch_scan_noalloc(const void *in, void *out, size_t n,
 	uint64_t *scratch, int *dev_status, int sm_count, cudaStream_t s) {
 	using Acc = typename std::conditional<(sizeof(OutT) <= 4), uint32_t,
 		uint64_t>::type;
-	const size_t tiles = (n + kTile - 1) / kTile;
+	using CFG = ScanBig<InT, OutT>;
+	const size_t tiles = (n + CFG::kTile - 1) / CFG::kTile;
 	TileStatus ts;
 	ts.words = scratch;
 	ts.counter = (uint32_t *)(scratch + (size_t)CLO_NOALLOC_MAX_TILES * 4);
@@ -488,13 +522,12 @@ cudaError_t launch_scan_noalloc(const void *in, void *out, size_t n,
 		tiles * Slots<Acc>::kPerTile * sizeof(uint64_t), s);
 	if (e == cudaSuccess) e = cudaMemsetAsync(ts.counter, 0, sizeof(uint64_t), s);
 	if (e != cudaSuccess) return e;
-	bool vec_ok = ((uintptr_t)in % 16 == 0) && ((uintptr_t)out % 16 == 0);
 	int per_sm = 1;
-	e = scan_prepare<InT, OutT>(&per_sm);
+	e = scan_prepare<InT, OutT, CFG>(&per_sm);
 	if (e != cudaSuccess) return e;
-	scan_lookback<InT, OutT><<<scan_grid(tiles, per_sm, sm_count), kThreads,
-		scan_smem<InT, OutT>(), s>>>(
-		(const InT *)in, (OutT *)out, n, ts, dev_status, vec_ok, -1, nullptr, nullptr);
+	scan_lookback<InT, OutT, CFG><<<scan_grid(tiles, per_sm, sm_count), CFG::kThreads, 0,
+		s>>>((const InT *)in, (OutT *)out, n, ts, dev_status, scan_vec(in, out), -1, nullptr,
+		nullptr);
 	count_launches(1);
 	return cudaGetLastError();
 }
