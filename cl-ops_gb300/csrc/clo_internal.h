@@ -133,6 +133,11 @@ cudaError_t radix_sort(const void *src, void *dst, void *vals, size_t n, int key
 cudaError_t radix_msd_partition(const void *keys_in, void *keys_out, size_t n, int key_bytes,
 	int sort_bits, uint32_t *counts, CCLContext *ctx, cudaStream_t s, GError **err);
 
+// Zeroes `bytes` (a multiple of 16) at a 16-byte aligned device address, as a
+// chained kernel (launch.h): a memset between two chained kernels would undo
+// the chaining.
+cudaError_t clear_chained(void *p, size_t bytes, cudaStream_t s);
+
 // Exclusive scan: out[i] = sum_{j<i} (sum type) in[j] modulo
 // 2^(8*out_bytes). in_type is an integer CloType, out_bytes in {1,2,4,8}.
 cudaError_t scan_exclusive(const void *in, void *out, size_t n,

@@ -253,8 +253,7 @@ scan_lookback(const InT *in, OutT *out, size_t n, TileStatus ts,
 	}
 }
 
-// Clears the tile statuses and the counter.
-__global__ void __launch_bounds__(256) scan_prep(uint4 *words, size_t count) {
+__global__ void __launch_bounds__(256) clear_words(uint4 *words, size_t count) {
 	dev::pdl_wait();
 	for (size_t i = blockIdx.x * (size_t)256 + threadIdx.x; i < count; i += (size_t)gridDim.x * 256)
 		words[i] = make_uint4(0, 0, 0, 0);
@@ -322,10 +321,7 @@ cudaError_t launch_scan_cfg(const void *in, void *out, size_t n, CCLContext *ctx
 		if (!tmp) return cudaErrorMemoryAllocation;
 		ts.words = (uint64_t *)tmp;
 		ts.counter = (uint32_t *)(tmp + status_bytes);
-		const size_t vecs = bytes / 16;
-		e = launch_chained(scan_prep, (unsigned)std::min<size_t>((vecs + 1023) / 1024, 64), 256, 0,
-			s, 1, (uint4 *)tmp, vecs);
-		count_launches(1);
+		e = clear_chained(tmp, bytes, s);
 	}
 	int per_sm = 1;
 	if (e == cudaSuccess) e = scan_prepare<InT, OutT, CFG>(&per_sm);
@@ -369,6 +365,13 @@ cudaError_t dispatch_out(const void *in, void *out, size_t n, int out_bytes,
 }
 
 }  // namespace
+
+cudaError_t clear_chained(void *p, size_t bytes, cudaStream_t s) {
+	const size_t vecs = bytes / 16;
+	count_launches(1);
+	return launch_chained(clear_words, (unsigned)std::min<size_t>((vecs + 1023) / 1024, 608), 256, 0,
+		s, 1, (uint4 *)p, vecs);
+}
 
 // Tile whose publication is withheld (-1: none). Only the watchdog test
 // sets it, through clo_gb300_debug_scan_withhold().

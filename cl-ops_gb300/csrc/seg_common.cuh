@@ -68,9 +68,14 @@ inline SegShape seg_shape(int v) {
 // Keys per thread and tile of the long-segment pass.
 template <typename K>
 constexpr int long_kpt(int idx) {
-	return sizeof(K) <= 4 ? (idx == 0 ? 56 : idx == 1 ? 48 : 40)
-						  : (idx == 0 ? 32 : idx == 1 ? 28 : 24);
+	return sizeof(K) <= 4 ? (idx == 0 ? 56 : idx == 1 ? 48 : idx == 2 ? 40 : 14)
+						  : (idx == 0 ? 32 : idx == 1 ? 28 : idx == 2 ? 24 : 8);
 }
+// Buffers that would not give every SM a tile of the shape's size take a
+// quarter of it (kSmallLong), whatever the shape: a 14336-key tile alone on
+// its SM takes 18 us a pass (100,000 keys in 100 segments, some of them long:
+// 95.6 us a sort, 58.7 with the small tiles).
+constexpr int kSmallLong = 3;
 template <typename K>
 constexpr uint32_t long_tile(int idx) {
 	return (uint32_t)(kLThreads * long_kpt<K>(idx));

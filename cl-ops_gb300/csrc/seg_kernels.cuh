@@ -9,6 +9,7 @@
 #include <type_traits>
 
 #include "dev_common.cuh"
+#include "launch.h"
 #include "seg_common.cuh"
 #include "timing.h"
 
@@ -36,8 +37,8 @@ struct CtaCfg {
 // peer masks, and a pass through shared memory back to index order.
 // Elements past the segment end are all-ones keys: they rank last in every
 // digit, so they stay behind the segment and are never written. Warps whose
-// keys all lie past the end take no part in the passes (their counts stay
-// zero), so a segment pays only for the warps it fills.
+// keys all lie past the end (fewer than 32 keys a warp) take no part in the
+// passes (their counts stay zero).
 template <typename K, int THREADS, int KPT, int RB>
 __global__ void __launch_bounds__(THREADS) seg_sort_cta(K *keys, const uint64_t *off,
 	const uint32_t *list, const uint32_t *count, int passes) {
@@ -59,21 +60,26 @@ __global__ void __launch_bounds__(THREADS) seg_sort_cta(K *keys, const uint64_t 
 	const uint32_t lt = dev::lanemask_lt();
 	for (int i = lane; i < R; i += 32) my_match[i] = 0;
 	auto dig = [](K key, int shift) { return (uint32_t)(key >> shift) & (uint32_t)(R - 1); };
+	dev::pdl_wait();
 	const uint32_t cnt = *count;
-	const uint32_t wb = (uint32_t)warp * (KPT * 32);
 
 	for (uint32_t li = blockIdx.x; li < cnt; li += gridDim.x) {
 		const uint32_t s = list[li];
 		const uint64_t base = off[s];
 		const uint32_t len = (uint32_t)(off[s + 1] - base);
+		// The segment's keys spread evenly over the warps, `rounds` a thread: a
+		// segment that fills part of the tile takes as many fewer rounds, not
+		// fewer warps (3 million keys in 1000 segments: 188 -> 155 us a sort).
+		const uint32_t rounds = (len + THREADS - 1) / THREADS;
+		const uint32_t wb = (uint32_t)warp * rounds * 32;
 		// Warps holding part of the segment, and the keys they hold.
 		const bool active = wb < len;
-		const uint32_t held = std::min<uint32_t>(TILE, (len + KPT * 32 - 1) / (KPT * 32) * (KPT * 32));
+		const uint32_t held = (len + rounds * 32 - 1) / (rounds * 32) * (rounds * 32);
 		K k[KPT];
 #pragma unroll
 		for (int j = 0; j < KPT; ++j) {
 			const uint32_t idx = wb + j * 32 + lane;
-			k[j] = idx < len ? keys[base + idx] : (K)~(K)0;
+			k[j] = (uint32_t)j < rounds && idx < len ? keys[base + idx] : (K)~(K)0;
 		}
 		for (int p = 0; p < passes; ++p) {
 			const int shift = p * RB;
@@ -81,7 +87,8 @@ __global__ void __launch_bounds__(THREADS) seg_sort_cta(K *keys, const uint64_t 
 			__syncwarp();
 			if (active) {
 #pragma unroll
-				for (int j = 0; j < KPT; ++j) atomicAdd(my_hist + dig(k[j], shift), 1u);
+				for (int j = 0; j < KPT; ++j)
+					if ((uint32_t)j < rounds) atomicAdd(my_hist + dig(k[j], shift), 1u);
 			}
 			__syncthreads();
 			// Digit totals (DPT consecutive digits per thread), the scan of
@@ -132,19 +139,21 @@ __global__ void __launch_bounds__(THREADS) seg_sort_cta(K *keys, const uint64_t 
 			if (active) {
 #pragma unroll
 				for (int j = 0; j < KPT; ++j) {
-					sk[dev::warp_rank_digit(my_match, my_hist, dig(k[j], shift), lane, lt)] = k[j];
+					if ((uint32_t)j < rounds)
+						sk[dev::warp_rank_digit(my_match, my_hist, dig(k[j], shift), lane, lt)] = k[j];
 				}
 			}
 			__syncthreads();
 			if (active) {
 #pragma unroll
-				for (int j = 0; j < KPT; ++j) k[j] = sk[wb + j * 32 + lane];
+				for (int j = 0; j < KPT; ++j)
+					if ((uint32_t)j < rounds) k[j] = sk[wb + j * 32 + lane];
 			}
 		}
 #pragma unroll
 		for (int j = 0; j < KPT; ++j) {
 			const uint32_t idx = wb + j * 32 + lane;
-			if (idx < len) keys[base + idx] = k[j];
+			if ((uint32_t)j < rounds && idx < len) keys[base + idx] = k[j];
 		}
 		__syncthreads();
 	}
@@ -226,6 +235,7 @@ seg_pass(const K *__restrict__ kin, K *__restrict__ kout, SegPassArgs a) {
 	const int shift = a.shift;
 #pragma unroll
 	for (int i = 0; i < HALF; ++i) s_cnt[seg_row(i) + pd] = 0;
+	dev::pdl_wait();
 	const uint32_t T = (uint32_t)(a.tstart[a.S] >> 32);
 	// Thread 0 takes the next tile and its descriptor (one round trip after
 	// the claim); after the first tile this overlaps the write-out.
@@ -413,10 +423,10 @@ cudaError_t launch_cta_class(K *keys, const uint64_t *off, const uint32_t *list,
 	uint32_t grid = (uint32_t)std::max(1, occ) * (uint32_t)ctx->sm_count;
 	if (grid > max_blocks) grid = std::max<uint32_t>(max_blocks, 1);
 	KernelTimer t("seg_sort_cta", s, 0.0);
-	kern<<<grid, THREADS, smem, s>>>(keys, off, list, count, sort_bits / RB);
+	e = launch_chained(kern, grid, THREADS, smem, s, 1, keys, off, list, count, sort_bits / RB);
 	t.stop();
 	count_launches(1);
-	return cudaGetLastError();
+	return e;
 }
 
 template <typename K, int THREADS, int KPT>
@@ -442,10 +452,10 @@ cudaError_t launch_pass_kpt(const K *src, K *dst, const SegPassArgs &pa, uint64_
 	const uint32_t grid = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(t_bound, 1),
 		(uint64_t)std::max(occ, 1) * ctx->sm_count);
 	KernelTimer t("seg_pass", s, 0.0);
-	kern<<<grid, kLThreads, smem, s>>>(src, dst, pa);
+	e = launch_chained(kern, grid, kLThreads, smem, s, 1, src, dst, pa);
 	t.stop();
 	count_launches(1);
-	return cudaGetLastError();
+	return e;
 }
 
 }  // namespace
@@ -488,6 +498,7 @@ cudaError_t seg_launch_pass(const SegShape &sh, const K *src, K *dst, const SegP
 	switch (sh.long_idx) {
 	case 1: return launch_pass_kpt<K, long_kpt<K>(1)>(src, dst, pa, t_bound, ctx, s);
 	case 2: return launch_pass_kpt<K, long_kpt<K>(2)>(src, dst, pa, t_bound, ctx, s);
+	case kSmallLong: return launch_pass_kpt<K, long_kpt<K>(kSmallLong)>(src, dst, pa, t_bound, ctx, s);
 	default: return launch_pass_kpt<K, long_kpt<K>(0)>(src, dst, pa, t_bound, ctx, s);
 	}
 }

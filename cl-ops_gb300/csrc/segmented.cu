@@ -33,6 +33,7 @@
 
 #include "clo_internal.h"
 #include "dev_common.cuh"
+#include "launch.h"
 #include "scan_status.cuh"
 #include "seg_common.cuh"
 #include "scan_tile.cuh"
@@ -83,6 +84,7 @@ struct ClassArgs {
 };
 
 __global__ void __launch_bounds__(256) seg_classify(ClassArgs a) {
+	dev::pdl_wait();
 	const uint32_t lane = threadIdx.x & 31u;
 	const uint32_t lt = dev::lanemask_lt();
 	const uint64_t warp_id = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
@@ -118,10 +120,70 @@ __global__ void __launch_bounds__(256) seg_classify(ClassArgs a) {
 	}
 }
 
+// The same for up to kClassifyOne segments in one CTA, which also scans the
+// tile counts (ca.tinfo receives the starts) and needs no cleared counters:
+// one launch for four.
+constexpr uint32_t kClassifyOne = 4096;
+__global__ void __launch_bounds__(1024) seg_classify_one(ClassArgs a) {
+	__shared__ uint32_t s_cnt[4];
+	__shared__ uint64_t s_tot[32], s_carry;
+	const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+	const uint32_t lt = dev::lanemask_lt();
+	if (tid < 4) s_cnt[tid] = 0;
+	if (tid == 0) s_carry = 0;
+	dev::pdl_wait();
+	if (tid < 16) a.counts[tid] = 0;  // the passes' tile counters among them
+	__syncthreads();
+	for (uint32_t s0 = 0; s0 <= a.S; s0 += 1024) {
+		const uint32_t s = s0 + tid;
+		int cls = -1;
+		uint64_t packed = 0;
+		if (s < a.S) {
+			const uint64_t len = checked_len(a.off, s, a.n_cap, a.dev_status);
+			if (len >= 2) {
+				if (len <= a.max_warp) cls = 0;
+				else if (len <= a.max_a) cls = 1;
+				else if (len <= a.max_b) cls = 2;
+				else {
+					cls = 3;
+					packed = (((len + a.large_tile - 1) / a.large_tile) << 32) | 1ull;
+				}
+			}
+		}
+#pragma unroll
+		for (int c = 0; c < 4; ++c) {
+			const uint32_t m = __ballot_sync(0xffffffffu, cls == c);
+			if (m) {
+				const int leader = __ffs(m) - 1;
+				uint32_t base = 0;
+				if ((int)lane == leader) base = atomicAdd(s_cnt + c, (uint32_t)__popc(m));
+				base = __shfl_sync(0xffffffffu, base, leader);
+				if (cls == c) a.lists[(size_t)c * a.S + base + __popc(m & lt)] = s;
+			}
+		}
+		uint64_t inc = packed;
+#pragma unroll
+		for (int d = 1; d < 32; d <<= 1) {
+			const uint64_t t = __shfl_up_sync(0xffffffffu, inc, d);
+			if (lane >= (uint32_t)d) inc += t;
+		}
+		if (lane == 31) s_tot[warp] = inc;
+		__syncthreads();
+		uint64_t before = s_carry + inc - packed;
+		for (uint32_t w = 0; w < warp; ++w) before += s_tot[w];
+		if (s <= a.S) a.tinfo[s] = before;
+		__syncthreads();
+		if (tid == 1023) s_carry = before + packed;
+		__syncthreads();
+	}
+	if (tid < 4) a.counts[tid] = s_cnt[tid];
+}
+
 // --------------------------------------------------------- warp class
 template <typename K>
 __global__ void __launch_bounds__(256) seg_sort_warp(K *keys, const uint64_t *off,
 	const uint32_t *list, const uint32_t *count, K mask) {
+	dev::pdl_wait();
 	const uint32_t lane = threadIdx.x & 31u;
 	const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
 	const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
@@ -166,6 +228,7 @@ __global__ void __launch_bounds__(256) seg_tiles(const uint64_t *off,
 	const uint64_t *tstart, const uint32_t *list, const uint32_t *count,
 	uint32_t *tile_seg, ulonglong2 *tile_span, uint2 *tile_x, uint32_t *seg_hist,
 	int passes, uint32_t *status0, uint32_t tile) {
+	dev::pdl_wait();
 	const uint32_t lane = threadIdx.x & 31u;
 	const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
 	const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
@@ -201,6 +264,7 @@ __global__ void __launch_bounds__(256) seg_upsweep(const K *keys, const uint64_t
 	__shared__ uint32_t h[PASSES * kRadix];
 	__shared__ uint64_t s_a, s_e;
 	__shared__ uint32_t s_lr;
+	dev::pdl_wait();
 	const uint32_t T = (uint32_t)(tstart[S] >> 32);
 	for (uint32_t t = blockIdx.x; t < T; t += gridDim.x) {
 		for (int i = threadIdx.x; i < PASSES * kRadix; i += blockDim.x) h[i] = 0;
@@ -244,6 +308,7 @@ template <typename K>
 __global__ void __launch_bounds__(256) seg_copy_large(K *dst, const K *src,
 	const uint64_t *off, const uint64_t *tstart, const uint32_t *tile_seg, uint32_t S,
 	uint32_t tile) {
+	dev::pdl_wait();
 	const uint32_t T = (uint32_t)(tstart[S] >> 32);
 	for (uint32_t t = blockIdx.x; t < T; t += gridDim.x) {
 		const uint32_t s = tile_seg[t];
@@ -259,6 +324,7 @@ __global__ void __launch_bounds__(256) seg_copy_large(K *dst, const K *src,
 template <typename K>
 __global__ void __launch_bounds__(256) seg_copy_short(K *dst, const K *src,
 	const uint64_t *off, const uint32_t *lists, const uint32_t *counts, uint32_t S) {
+	dev::pdl_wait();
 	const uint32_t lane = threadIdx.x & 31u;
 	const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
 	const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
@@ -272,18 +338,18 @@ __global__ void __launch_bounds__(256) seg_copy_short(K *dst, const K *src,
 }
 
 template <typename K>
-void launch_seg_upsweep(int passes, uint32_t grid, cudaStream_t s, const K *keys,
+cudaError_t launch_seg_upsweep(int passes, uint32_t grid, cudaStream_t s, const K *keys,
 	const uint64_t *off, const uint64_t *tstart, const uint32_t *tile_seg, uint32_t S,
 	uint32_t *seg_hist, uint32_t tile) {
 	switch (passes) {
-	case 1: seg_upsweep<K, 1><<<grid, 256, 0, s>>>(keys, off, tstart, tile_seg, S, seg_hist, tile); break;
-	case 2: seg_upsweep<K, 2><<<grid, 256, 0, s>>>(keys, off, tstart, tile_seg, S, seg_hist, tile); break;
-	case 3: seg_upsweep<K, 3><<<grid, 256, 0, s>>>(keys, off, tstart, tile_seg, S, seg_hist, tile); break;
-	case 4: seg_upsweep<K, 4><<<grid, 256, 0, s>>>(keys, off, tstart, tile_seg, S, seg_hist, tile); break;
-	case 5: seg_upsweep<K, 5><<<grid, 256, 0, s>>>(keys, off, tstart, tile_seg, S, seg_hist, tile); break;
-	case 6: seg_upsweep<K, 6><<<grid, 256, 0, s>>>(keys, off, tstart, tile_seg, S, seg_hist, tile); break;
-	case 7: seg_upsweep<K, 7><<<grid, 256, 0, s>>>(keys, off, tstart, tile_seg, S, seg_hist, tile); break;
-	default: seg_upsweep<K, 8><<<grid, 256, 0, s>>>(keys, off, tstart, tile_seg, S, seg_hist, tile); break;
+	case 1: return launch_chained(seg_upsweep<K, 1>, grid, 256, 0, s, 1, keys, off, tstart, tile_seg, S, seg_hist, tile);
+	case 2: return launch_chained(seg_upsweep<K, 2>, grid, 256, 0, s, 1, keys, off, tstart, tile_seg, S, seg_hist, tile);
+	case 3: return launch_chained(seg_upsweep<K, 3>, grid, 256, 0, s, 1, keys, off, tstart, tile_seg, S, seg_hist, tile);
+	case 4: return launch_chained(seg_upsweep<K, 4>, grid, 256, 0, s, 1, keys, off, tstart, tile_seg, S, seg_hist, tile);
+	case 5: return launch_chained(seg_upsweep<K, 5>, grid, 256, 0, s, 1, keys, off, tstart, tile_seg, S, seg_hist, tile);
+	case 6: return launch_chained(seg_upsweep<K, 6>, grid, 256, 0, s, 1, keys, off, tstart, tile_seg, S, seg_hist, tile);
+	case 7: return launch_chained(seg_upsweep<K, 7>, grid, 256, 0, s, 1, keys, off, tstart, tile_seg, S, seg_hist, tile);
+	default: return launch_chained(seg_upsweep<K, 8>, grid, 256, 0, s, 1, keys, off, tstart, tile_seg, S, seg_hist, tile);
 	}
 }
 
@@ -291,7 +357,8 @@ template <typename K>
 cudaError_t seg_sort_typed(K *keys, uint64_t n_cap, const uint64_t *off, uint32_t S,
 	int sort_bits, int variant, CCLContext *ctx, cudaStream_t s, GError **err,
 	K *alt_ext, bool *in_alt) {
-	const SegShape sh = seg_shape(variant);
+	SegShape sh = seg_shape(variant);
+	if (n_cap < (uint64_t)ctx->sm_count * long_tile<K>(sh.long_idx)) sh.long_idx = kSmallLong;
 	const uint32_t LTILE = long_tile<K>(sh.long_idx);
 	const int passes = sort_bits / kRadixBits;
 	if (in_alt) *in_alt = false;
@@ -329,7 +396,8 @@ cudaError_t seg_sort_typed(K *keys, uint64_t n_cap, const uint64_t *off, uint32_
 	uint32_t *st[2] = {(uint32_t *)(tmp + off_st0), (uint32_t *)(tmp + off_st1)};
 	K *alt = alt_ext ? alt_ext : (K *)(tmp + off_alt);
 	unsigned launches = 0;
-	cudaError_t e = cudaMemsetAsync(counts, 0, 64, s);
+	const bool one = S <= kClassifyOne;
+	cudaError_t e = one ? cudaSuccess : clear_chained(counts, 64, s);
 	if (e == cudaSuccess) {
 		ClassArgs ca;
 		ca.off = off;
@@ -341,15 +409,15 @@ cudaError_t seg_sort_typed(K *keys, uint64_t n_cap, const uint64_t *off, uint32_
 		ca.large_tile = LTILE;
 		ca.lists = lists;
 		ca.counts = counts;
-		ca.tinfo = tinfo;
+		ca.tinfo = one ? tstart : tinfo;
 		ca.dev_status = ctx->d_status;
 		const uint32_t grid = (uint32_t)std::min<uint64_t>(((uint64_t)S + 1 + 255) / 256,
 			(uint64_t)ctx->sm_count * 8);
-		seg_classify<<<grid, 256, 0, s>>>(ca);
+		e = one ? launch_chained(seg_classify_one, 1, 1024, 0, s, 1, ca)
+				: launch_chained(seg_classify, grid, 256, 0, s, 1, ca);
 		launches++;
-		e = cudaGetLastError();
 	}
-	if (e == cudaSuccess)
+	if (e == cudaSuccess && !one && L_bound > 0)
 		e = scan_exclusive(tinfo, tstart, (size_t)S + 1, CLO_ULONG, 8, ctx, s, err);
 	const K mask = sort_bits >= (int)(8 * sizeof(K)) ? (K)~(K)0
 		: (K)(((K)1 << sort_bits) - 1);
@@ -357,10 +425,9 @@ cudaError_t seg_sort_typed(K *keys, uint64_t n_cap, const uint64_t *off, uint32_
 		const uint32_t grid = (uint32_t)std::min<uint64_t>(((uint64_t)S + 7) / 8,
 			(uint64_t)ctx->sm_count * 8);
 		KernelTimer t("seg_sort_warp", s, 0.0);
-		seg_sort_warp<K><<<grid, 256, 0, s>>>(keys, off, lists, counts, mask);
+		e = launch_chained(seg_sort_warp<K>, grid, 256, 0, s, 1, keys, off, lists, counts, mask);
 		t.stop();
 		launches++;
-		e = cudaGetLastError();
 	}
 	if (e == cudaSuccess)
 		e = seg_launch_cta_classes<K>(sh, keys, off, lists, counts, S, sort_bits, n_cap, ctx, s);
@@ -369,20 +436,18 @@ cudaError_t seg_sort_typed(K *keys, uint64_t n_cap, const uint64_t *off, uint32_
 		{
 			const uint32_t grid = (uint32_t)std::min<uint64_t>((L_bound + 7) / 8,
 				(uint64_t)ctx->sm_count * 8);
-			seg_tiles<<<grid, 256, 0, s>>>(off, tstart, list3, counts + 3, tile_seg,
+			e = launch_chained(seg_tiles, grid, 256, 0, s, 1, off, tstart, list3, counts + 3, tile_seg,
 				tile_span, tile_x, seg_hist, passes, st[0], LTILE);
 			launches++;
-			e = cudaGetLastError();
 		}
 		if (e == cudaSuccess) {
 			const uint32_t grid = (uint32_t)std::min<uint64_t>(T_bound,
 				(uint64_t)ctx->sm_count * 8);
 			KernelTimer t("seg_upsweep", s, 0.0);
-			launch_seg_upsweep<K>(passes, grid, s, keys, off, tstart, tile_seg, S, seg_hist,
+			e = launch_seg_upsweep<K>(passes, grid, s, keys, off, tstart, tile_seg, S, seg_hist,
 				LTILE);
 			t.stop();
 			launches++;
-			e = cudaGetLastError();
 		}
 		K *src = keys, *dst = alt;
 		for (int p = 0; p < passes && e == cudaSuccess; ++p) {
@@ -408,16 +473,15 @@ cudaError_t seg_sort_typed(K *keys, uint64_t n_cap, const uint64_t *off, uint32_
 			// the short ones, sorted in place, are copied there.
 			const uint32_t grid = (uint32_t)std::min<uint64_t>(((uint64_t)S + 7) / 8,
 				(uint64_t)ctx->sm_count * 8);
-			seg_copy_short<K><<<grid, 256, 0, s>>>(alt, keys, off, lists, counts, S);
+			e = launch_chained(seg_copy_short<K>, grid, 256, 0, s, 1, alt, keys, off, lists, counts, S);
 			launches++;
-			e = cudaGetLastError();
 			*in_alt = true;
 		} else if (e == cudaSuccess && (passes & 1)) {
 			const uint32_t grid = (uint32_t)std::min<uint64_t>(T_bound,
 				(uint64_t)ctx->sm_count * 8);
-			seg_copy_large<K><<<grid, 256, 0, s>>>(keys, alt, off, tstart, tile_seg, S, LTILE);
+			e = launch_chained(seg_copy_large<K>, grid, 256, 0, s, 1, keys, alt, off, tstart, tile_seg, S,
+				LTILE);
 			launches++;
-			e = cudaGetLastError();
 		}
 	}
 	count_launches(launches);
@@ -431,6 +495,7 @@ cudaError_t seg_sort_typed(K *keys, uint64_t n_cap, const uint64_t *off, uint32_
 // elements).
 __global__ void __launch_bounds__(256) seg_heads(const uint64_t *off, uint32_t S,
 	uint64_t n_cap, uint32_t *bits, int *dev_status) {
+	dev::pdl_wait();
 	const uint64_t end = off[S];
 	for (uint64_t s = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; s < S;
 		 s += (uint64_t)gridDim.x * blockDim.x) {
@@ -473,6 +538,7 @@ seg_scan_lookback(const InT *__restrict__ in, OutT *__restrict__ out, uint64_t n
 		(kBlocks * padded<InT>() * sizeof(InT) + padded<OutT>() * sizeof(OutT)));
 	OutT *s_out = reinterpret_cast<OutT *>(s_in + kBlocks * padded<InT>());
 	auto full_tile = [&](uint32_t t) { return vec_ok && (uint64_t)(t + 1) * kTile <= n; };
+	dev::pdl_wait();
 	if (tid == 0) {
 		s_tile = atomicAdd(ts.counter, 1u);
 		s_lo = off[0];
@@ -751,23 +817,22 @@ cudaError_t launch_seg_scan(const void *in, void *out, uint64_t n_cap,
 	lb::TileStatus ts;
 	ts.words = (uint64_t *)(tmp + bm_bytes);
 	ts.counter = (uint32_t *)(tmp + bm_bytes + st_bytes);
-	e = cudaMemsetAsync(tmp, 0, total, s);
+	e = clear_chained(tmp, total, s);
 	if (e == cudaSuccess) {
 		const uint32_t grid = (uint32_t)std::min<uint64_t>(((uint64_t)S + 255) / 256,
 			(uint64_t)ctx->sm_count * 8);
-		seg_heads<<<std::max<uint32_t>(grid, 1), 256, 0, s>>>(off, S, n_cap, bits,
+		e = launch_chained(seg_heads, std::max<uint32_t>(grid, 1), 256, 0, s, 1, off, S, n_cap, bits,
 			ctx->d_status);
-		e = cudaGetLastError();
 	}
 	const bool vec_ok = ((uintptr_t)in % 16 == 0) && ((uintptr_t)out % 16 == 0);
 	if (e == cudaSuccess) {
 		const unsigned grid = (unsigned)std::max<uint64_t>(1,
 			std::min<uint64_t>(tiles, (uint64_t)per_sm * ctx->sm_count));
 		KernelTimer t("seg_scan_lookback", s, (double)n_cap * (sizeof(InT) + sizeof(OutT)));
-		seg_scan_lookback<InT, OutT><<<grid, scantile::kThreads, scantile::scan_smem<InT, OutT>(), s>>>(
-			(const InT *)in, (OutT *)out, n_cap, bits, off, S, ts, ctx->d_status, vec_ok);
+		e = launch_chained(seg_scan_lookback<InT, OutT>, grid, scantile::kThreads,
+			scantile::scan_smem<InT, OutT>(), s, 1, (const InT *)in, (OutT *)out, n_cap, bits, off, S,
+			ts, ctx->d_status, vec_ok);
 		t.stop();
-		e = cudaGetLastError();
 	}
 	count_launches(2);
 	tmp_free(tmp, s);

@@ -48,3 +48,28 @@ def test_shape_edges(clops, ctx, queue, in_type, in_dt, sum_type, sum_dt, n):
     for off_in, off_out in ((0, 0), (16, 32), (0, 16), (a.itemsize, 0)):
         got = _scan_at(clops, ctx, queue, a, in_type, sum_type, sum_dt, off_in, off_out)
         np.testing.assert_array_equal(got, ref)
+
+
+@pytest.mark.parametrize("segments", [1, 1023, 1024, 4096, 4097])
+@pytest.mark.parametrize("code,dt", [(5, np.uint32), (7, np.uint64)])
+def test_segment_counts_around_the_one_cta_classification(clops, ctx, queue, segments, code, dt):
+    """Segments of every class (and one long enough for several tiles) by
+    number: one CTA classifies up to 4096; the buffer is small enough for the
+    quarter-size tiles of the long segments."""
+    lens = (splitmix64(segments, segments) % np.uint64(70)).astype(np.int64)
+    lens[:: max(1, segments // 7)] = 3000
+    lens[0] = 30000
+    lens[-1] = max(lens[-1], 9001)
+    off = np.zeros(segments + 1, dtype=np.uint64)
+    off[1:] = np.cumsum(lens).astype(np.uint64)
+    n = int(off[-1])
+    a = splitmix64(5, n).astype(dt)
+    s = clops.Sorter(ctx, "satradix", code)
+    b = clops.Buffer.from_array(ctx, queue, a)
+    ob = clops.Buffer.from_array(ctx, queue, off)
+    clops.wait(s.sort_segmented_device(queue, b, ob, segments))
+    got = b.read(queue, dt, n)
+    seg = np.repeat(np.arange(segments), lens)
+    np.testing.assert_array_equal(got, a[np.lexsort((a, seg))])
+    for x in (b, ob, s):
+        x.destroy()
