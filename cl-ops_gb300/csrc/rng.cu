@@ -12,13 +12,14 @@
 // Fill (the draw loop of src/benchmarks/clo_rng_bench.c:302-324 with the
 // kernel of clo_rng_bench.cl:23-37, moved on device): out[r * count + i]
 // = next(state i) >> (32 - bits), or % maxint, for r = 0..draws-1. Each
-// thread keeps 4 consecutive states in registers for all draws and writes
-// one 16-byte vector per draw, so the states are read and written once.
+// thread keeps one state, or four consecutive ones, in registers for all
+// draws, so the states are read and written once.
 //
 // HBM roofline: 4 B per draw + 2 x state size per state.
 #include "clo_internal.h"
 #include "clo_rng_device.cuh"
 #include "dev_common.cuh"
+#include "launch.h"
 #include "timing.h"
 
 namespace clo {
@@ -128,63 +129,74 @@ struct Gen<RNG_TAUSLCG> {
 
 constexpr int kFillThreads = 256;
 
-// 4 consecutive states per thread; one uint4 store per draw.
-template <int GEN, bool MAXINT>
+// V consecutive states per thread (4: one 16-byte store per draw; 1: coalesced
+// 4-byte stores, any count and alignment).
+template <int GEN, bool MAXINT, int V>
 __global__ void __launch_bounds__(kFillThreads)
 rng_fill_kernel(typename Gen<GEN>::S *__restrict__ states, size_t count,
-	uint32_t *__restrict__ out, size_t draws, uint32_t shift, uint32_t maxint,
-	bool vec) {
+	uint32_t *__restrict__ out, size_t draws, uint32_t shift, uint32_t maxint) {
 	using S = typename Gen<GEN>::S;
 	const size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-	const size_t i0 = q * 4;
+	const size_t i0 = q * V;
+	dev::pdl_wait();
 	if (i0 >= count) return;
 	auto emit = [&](uint32_t v) -> uint32_t {
 		return MAXINT ? v % maxint : (v >> shift);
 	};
-	if (vec) {
-		S s0 = states[i0], s1 = states[i0 + 1], s2 = states[i0 + 2], s3 = states[i0 + 3];
-		uint4 *o = reinterpret_cast<uint4 *>(out) + q;
-		const size_t row = count / 4;
-		for (size_t r = 0; r < draws; ++r) {
-			uint4 v;
-			v.x = emit(Gen<GEN>::next(s0));
-			v.y = emit(Gen<GEN>::next(s1));
-			v.z = emit(Gen<GEN>::next(s2));
-			v.w = emit(Gen<GEN>::next(s3));
-			dev::st_stream_v4(o + r * row, v);
-		}
-		states[i0] = s0;
-		states[i0 + 1] = s1;
-		states[i0 + 2] = s2;
-		states[i0 + 3] = s3;
-	} else {
-		for (size_t i = i0; i < i0 + 4 && i < count; ++i) {
-			S s = states[i];
-			for (size_t r = 0; r < draws; ++r) out[r * count + i] = emit(Gen<GEN>::next(s));
-			states[i] = s;
-		}
+	S s[V];
+#pragma unroll
+	for (int k = 0; k < V; ++k) s[k] = states[i0 + k];
+	uint32_t *o = out + i0;
+#pragma unroll 4
+	for (size_t r = 0; r < draws; ++r, o += count) {
+		uint32_t v[V];
+#pragma unroll
+		for (int k = 0; k < V; ++k) v[k] = emit(Gen<GEN>::next(s[k]));
+		if constexpr (V == 4)
+			dev::st_stream_v4(reinterpret_cast<uint4 *>(o), make_uint4(v[0], v[1], v[2], v[3]));
+		else
+			__stcs(o, v[0]);
 	}
+#pragma unroll
+	for (int k = 0; k < V; ++k) states[i0 + k] = s[k];
 }
+
+template <int GEN, bool MAXINT, int V>
+cudaError_t launch_fill(void *states, size_t count, uint32_t *out, size_t draws, uint32_t shift,
+	unsigned maxint, cudaStream_t s) {
+	using S = typename Gen<GEN>::S;
+	const size_t threads = (count + V - 1) / V;
+	return launch_chained(rng_fill_kernel<GEN, MAXINT, V>,
+		(unsigned)((threads + kFillThreads - 1) / kFillThreads), kFillThreads, 0, s, 1, (S *)states,
+		count, out, draws, shift, maxint);
+}
+
+// Counts from which a thread takes four states (whole rows of 16-byte stores
+// need count % 4 == 0 and an aligned output too); below, one state a thread
+// fills the SMs better. us, four / one: mwc64x 65536 x 64 5.8 / 4.0, 262144 x
+// 32 6.6 / 6.2, 2^20 x 32 21.4 / 19.5, 2^22 x 32 88.2 / 90.3; parkmiller
+// 262144 x 32 6.6 / 6.8, 2^20 x 32 20.1 / 22.8. Counts that are no multiple of
+// four (2^22 - 1 mwc64x x 32): 138 us, whose rows' stores meet the 32-byte
+// sectors unaligned; 524 with four states a thread one after the other.
+template <int GEN>
+constexpr size_t kVecMin = GEN == RNG_PARKMILLER ? (size_t)1 << 18 : (size_t)1 << 21;
 
 template <int GEN>
 cudaError_t fill_gen(void *states, size_t count, uint32_t *out, size_t draws,
 	unsigned bits, unsigned maxint, cudaStream_t s) {
 	using S = typename Gen<GEN>::S;
-	size_t threads = (count + 3) / 4;
-	unsigned blocks = (unsigned)((threads + kFillThreads - 1) / kFillThreads);
-	uint32_t shift = 32u - bits;
-	// Whole rows of 16-byte stores need count % 4 == 0 and an aligned out.
-	bool vec = (count % 4) == 0 && ((uintptr_t)out % 16) == 0;
+	const uint32_t shift = 32u - bits;
+	const bool vec = (count % 4) == 0 && ((uintptr_t)out % 16) == 0 &&
+		count >= kVecMin<GEN>;
 	KernelTimer t("rng_fill", s, (double)count * (4.0 * draws + 2.0 * sizeof(S)));
-	if (maxint)
-		rng_fill_kernel<GEN, true><<<blocks, kFillThreads, 0, s>>>((S *)states, count,
-			out, draws, shift, maxint, vec);
-	else
-		rng_fill_kernel<GEN, false><<<blocks, kFillThreads, 0, s>>>((S *)states, count,
-			out, draws, shift, maxint, vec);
+	const cudaError_t e = maxint
+		? (vec ? launch_fill<GEN, true, 4>(states, count, out, draws, shift, maxint, s)
+			   : launch_fill<GEN, true, 1>(states, count, out, draws, shift, maxint, s))
+		: (vec ? launch_fill<GEN, false, 4>(states, count, out, draws, shift, maxint, s)
+			   : launch_fill<GEN, false, 1>(states, count, out, draws, shift, maxint, s));
 	t.stop();
 	count_launches(1);
-	return cudaGetLastError();
+	return e;
 }
 
 }  // namespace
