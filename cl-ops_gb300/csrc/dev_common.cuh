@@ -237,5 +237,19 @@ __device__ __forceinline__ uint32_t unit_rank_digit(uint32_t *w, uint32_t l16,
 	return (v >> 16) + below;
 }
 
+// The same for the lanes where `ok` holds; the others only synchronise.
+__device__ __forceinline__ uint32_t unit_rank_digit_if(bool ok, uint32_t *w, uint32_t l16,
+	uint32_t lt16) {
+	if (ok) atomicOr(w, 1u << l16);
+	__syncwarp();
+	const uint32_t v = ok ? *w : 0u;
+	__syncwarp();
+	const uint32_t peers = v & 0xFFFFu;
+	const uint32_t below = __popc(peers & lt16);
+	if (ok && below == 0) *w = (v & 0xFFFF0000u) + ((uint32_t)__popc(peers) << 16);
+	__syncwarp();
+	return (v >> 16) + below;
+}
+
 }  // namespace dev
 }  // namespace clo

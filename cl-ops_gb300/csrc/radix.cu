@@ -38,15 +38,11 @@ cudaError_t radix_sort(const void *src, void *dst, void *vals, size_t n, int key
 	if (none) return cudaSuccess;
 	// Small whole-key sorts without values: equal keys are the same bits, so
 	// any sort gives the stable one's result, and the bitonic tile kernel does
-	// up to 2^15 elements in one launch and no scratch (us, bitonic / radix:
-	// 2^10 u32 5.0 / 15.2, 2^15 u32 15 / 25, 2^15 u64 33 / 45, 2^12 u16 7.8 /
-	// 12; from 2^14 u16 and 2^13 u8 the radix sort's few passes are faster).
-	if (val_bytes == 0 && sort_bits == 8 * key_bytes &&
-		n <= ((size_t)1 << (key_bytes >= 4 ? 15 : key_bytes == 2 ? 13 : 12)))
-		return bitonic_sort(src, dst, n,
-			key_bytes == 8 ? CLO_ULONG : key_bytes == 4 ? CLO_UINT : key_bytes == 2 ? CLO_USHORT
-																				  : CLO_UCHAR,
-			4, 0, ctx, s, err);
+	// up to 2^15 elements in one launch and no scratch (us, bitonic / the radix
+	// sort's best: 2^10 u32 5.1 / 8.2, 2^12 6.5 / 11, 2^15 15 / 25, 2^10 u64 9.9
+	// / 15, 2^15 33 / 44; keys of one and two bytes are faster by radix).
+	if (val_bytes == 0 && key_bytes >= 4 && sort_bits == 8 * key_bytes && n <= ((size_t)1 << 15))
+		return bitonic_sort(src, dst, n, key_bytes == 8 ? CLO_ULONG : CLO_UINT, 4, 0, ctx, s, err);
 	switch (key_bytes) {
 	case 1: return radix::sort<uint8_t>(src, dst, vals, n, val_bytes, sort_bits, ctx, s, err);
 	case 2: return radix::sort<uint16_t>(src, dst, vals, n, val_bytes, sort_bits, ctx, s, err);

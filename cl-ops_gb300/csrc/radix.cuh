@@ -266,6 +266,49 @@ radix_upsweep_w(const K *__restrict__ keys, size_t n, int base_shift, UpTail tai
 	upsweep_tail<PASSES, kUpwThreads>(tail);
 }
 
+// ------------------------------------------------------- one-byte keys
+// Writes the sorted bytes from the digit bases: byte i is the digit whose run
+// holds i. A thread writes 16 bytes at a time, found by a search in the 256
+// bases. Bound by the writes: a sort reads and writes each key once (2^26
+// keys: 37 us against 217 with a ranked pass and, in place, a copy back).
+constexpr int kFillBytesThreads = 256;
+__global__ void __launch_bounds__(kFillBytesThreads)
+radix_fill_bytes(uint8_t *out, size_t n, const uint32_t *base) {
+	__shared__ uint32_t s_base[kRadix + 1];
+	dev::pdl_wait();
+	s_base[threadIdx.x] = base[threadIdx.x];
+	if (threadIdx.x == 0) s_base[kRadix] = (uint32_t)n;
+	__syncthreads();
+	const bool vec = ((uintptr_t)out % 16) == 0;
+	const size_t stride = (size_t)gridDim.x * kFillBytesThreads * 16;
+	for (size_t i0 = (blockIdx.x * (size_t)kFillBytesThreads + threadIdx.x) * 16; i0 < n; i0 += stride) {
+		// The last digit whose base is at most i0.
+		uint32_t d = 0;
+#pragma unroll
+		for (uint32_t step = kRadix / 2; step; step >>= 1)
+			if (s_base[d + step] <= i0) d += step;
+		const size_t end = i0 + 16 < n ? i0 + 16 : n;
+		uint32_t w[4];
+		if (s_base[d + 1] >= end) {
+			w[0] = w[1] = w[2] = w[3] = d * 0x01010101u;
+		} else {
+#pragma unroll
+			for (int q = 0; q < 16; ++q) {
+				while (i0 + q < end && s_base[d + 1] <= i0 + q) ++d;
+				if (q % 4 == 0) w[q / 4] = 0;
+				w[q / 4] |= d << (8 * (q % 4));
+			}
+		}
+		if (vec && end - i0 == 16) {
+			*reinterpret_cast<uint4 *>(out + i0) = make_uint4(w[0], w[1], w[2], w[3]);
+		} else {
+#pragma unroll
+			for (int q = 0; q < 16; ++q)
+				if (i0 + q < end) out[i0 + q] = (uint8_t)(w[q / 4] >> (8 * (q % 4)));
+		}
+	}
+}
+
 // ------------------------------------------------- pass state and lookback
 template <typename K, typename V>
 struct PassArgs {
@@ -676,6 +719,193 @@ radix_pass_tiles(const __grid_constant__ PassArgs<K, V> a, uint32_t num_tiles) {
 	}
 }
 
+// ------------------------------------------------- small sorts in a cluster
+// Small sorts in one launch: a cluster of CL CTAs (one for the smallest) holds the keys, CTA c the slice
+// [c * slice, (c + 1) * slice) in its shared memory. Per digit: keys into
+// registers by half-warp units as in radix_pass_tiles, unit counts, the
+// CTA's digit totals read by every CTA through distributed shared memory,
+// each unit's first position of every digit, ranks, and each key (and value)
+// stored straight to its place in the slice that holds it. Two cluster
+// barriers a digit take the place of a launch, a tile claim, a load, a
+// lookback and a store to memory. A digit that holds every key is skipped.
+constexpr int kClThreads = 512, kClUnits = kClThreads / 16, kClRounds = 16;
+// Largest sort of one CTA and of a cluster of eight (0: the multi-launch sort
+// or, for whole 4- and 8-byte keys, the bitonic tiles are faster). us a sort,
+// this / multi-launch, pairs with two client copies: (u32, u32) 2^10 15.8 /
+// 23.6, 2^12 20.5 / 31.8, 2^14 30.7 / 33.8, 2^15 41 / 36; (u64, u64) 2^12 34.8
+// / 53.3, 2^14 51.7 / 59.4, 2^15 75.8 / 59.4; u16 keys 2^13 8.7 / 12.2; u8 keys
+// 2^13 5.0 / 7.9. At 2^12 one CTA and eight are equal.
+template <typename K>
+constexpr size_t kOneCtaKeys = sizeof(K) <= 2 ? 8192 : 4096;
+template <typename K, bool HAS_V>
+constexpr size_t kClusterKeys = HAS_V || sizeof(K) == 8 ? 16384 : 0;
+
+template <typename K, typename V, bool HAS_V>
+constexpr size_t cluster_smem(size_t slice) {
+	return ((size_t)(kClUnits + kClUnits / 2) * kRowWords + 2 * kRadix) * 4 +
+		(slice * (sizeof(K) + (HAS_V ? sizeof(V) : 0)) + 15) / 16 * 16;
+}
+
+template <typename K, typename V, bool HAS_V, int CL>
+__global__ void __launch_bounds__(kClThreads, 1)
+radix_cluster(const K *kin, K *kout, const V *vin, V *vout, uint32_t n, uint32_t rounds,
+	int passes) {
+	constexpr int HALF = kClUnits / 2, R = kClRounds;
+	extern __shared__ __align__(16) unsigned char cl_shared[];
+	uint32_t *s_rank = reinterpret_cast<uint32_t *>(cl_shared);  // [units] rows
+	uint32_t *s_cnt = s_rank + kClUnits * kRowWords;             // [HALF] rows
+	uint32_t *s_own = s_cnt + HALF * kRowWords;                  // [2][256] digit totals
+	const uint32_t slice = rounds * kClThreads;
+	// 8-byte parts first, so that both are aligned (a slice is a multiple of
+	// 512 elements).
+	unsigned char *s_data = reinterpret_cast<unsigned char *>(s_own + 2 * kRadix);
+	K *s_key = reinterpret_cast<K *>(s_data);
+	V *s_val = reinterpret_cast<V *>(s_data + (size_t)slice * sizeof(K));
+	__shared__ uint32_t s_scan[8];
+
+	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+	const int unit = 2 * warp + (lane >> 4);
+	const uint32_t l16 = lane & 15, lt16 = (1u << l16) - 1u;
+	const uint32_t rank = CL > 1 ? dev::cluster_rank() : 0u;
+	uint32_t *my_rank = s_rank + row_of(unit);
+	uint32_t *my_cnt = s_cnt + row_of(unit % HALF);
+	const uint32_t cnt_inc = 1u << ((unit / HALF) * 16);
+	const bool owner = tid < kRadix;
+	const uint32_t first = rank * slice;                     // of this CTA's slice
+	const uint32_t local = (uint32_t)unit * 16 * rounds + l16;  // of this thread, round 0
+	const uint32_t held = first < n ? std::min<uint32_t>(slice, n - first) : 0;
+	const uint32_t per_slice = (uint32_t)((1ull << 32) / slice) + 1u;  // pos / slice as a product
+	auto barrier = [] {
+		if constexpr (CL > 1) {
+			dev::cluster_arrive();
+			dev::cluster_wait();
+		} else {
+			__syncthreads();
+		}
+	};
+	K k[R];
+	V v[HAS_V ? R : 1];
+	dev::pdl_wait();
+#pragma unroll
+	for (int j = 0; j < R; ++j) {
+		const uint32_t i = local + j * 16;
+		const bool ok = (uint32_t)j < rounds && i < held;
+		k[j] = ok ? kin[first + i] : (K)0;
+		if constexpr (HAS_V) v[j] = ok ? vin[first + i] : (V)0;
+	}
+	bool moved = false;  // the slice is in shared memory
+	for (int p = 0; p < passes; ++p) {
+		const int shift = p * kRadixBits;
+		uint32_t *own = s_own + (p & 1) * kRadix;
+		if (owner)
+#pragma unroll
+			for (int i = 0; i < HALF; ++i) s_cnt[row_of(i) + tid] = 0;
+		__syncthreads();
+#pragma unroll
+		for (int j = 0; j < R; ++j)
+			if ((uint32_t)j < rounds && local + j * 16 < held)
+				atomicAdd(my_cnt + digit_of(k[j], shift), cnt_inc);
+		__syncthreads();
+		uint32_t c[HALF];
+		uint32_t mine = 0;
+		if (owner) {
+#pragma unroll
+			for (int i = 0; i < HALF; ++i) {
+				c[i] = s_cnt[row_of(i) + tid];
+				mine += (c[i] & 0xFFFFu) + (c[i] >> 16);
+			}
+			own[tid] = mine;
+		}
+		// Every CTA's totals are out, and every CTA has its keys in registers.
+		barrier();
+		uint32_t total = mine, before = 0, inc = 0;
+		if (owner) {
+			if constexpr (CL > 1) {
+				const uint32_t a = dev::smem_u32(own + tid);
+				total = 0;
+#pragma unroll
+				for (int r = 0; r < CL; ++r) {
+					const uint32_t x = dev::ld_dsmem<uint32_t>(dev::map_shared(a, r));
+					total += x;
+					if ((uint32_t)r < rank) before += x;
+				}
+			}
+			inc = total;
+#pragma unroll
+			for (int d = 1; d < 32; d <<= 1) {
+				const uint32_t t = __shfl_up_sync(0xffffffffu, inc, d);
+				if (lane >= d) inc += t;
+			}
+			if (lane == 31) s_scan[warp] = inc;
+		}
+		// (The same in every CTA.) One digit holds every key: nothing moves.
+		if (__syncthreads_or(owner && total == n)) continue;
+		if (owner) {
+			uint32_t at = inc - total + before;
+			for (int w = 0; w < warp; ++w) at += s_scan[w];
+#pragma unroll
+			for (int i = 0; i < HALF; ++i) {
+				s_rank[row_of(i) + tid] = at << 16;
+				at += c[i] & 0xFFFFu;
+			}
+#pragma unroll
+			for (int i = 0; i < HALF; ++i) {
+				s_rank[row_of(i + HALF) + tid] = at << 16;
+				at += c[i] >> 16;
+			}
+		}
+		__syncthreads();
+#pragma unroll
+		for (int j = 0; j < R; ++j) {
+			if ((uint32_t)j < rounds) {
+				const bool ok = local + j * 16 < held;
+				const uint32_t pos = dev::unit_rank_digit_if(ok, my_rank + digit_of(k[j], shift), l16,
+					lt16);
+				if (ok) {
+					if constexpr (CL > 1) {
+						const uint32_t to = __umulhi(pos, per_slice), o = pos - to * slice;
+						dev::st_dsmem<K>(dev::map_shared(dev::smem_u32(s_key + o), to), k[j]);
+						if constexpr (HAS_V)
+							dev::st_dsmem<V>(dev::map_shared(dev::smem_u32(s_val + o), to), v[j]);
+					} else {
+						s_key[pos] = k[j];
+						if constexpr (HAS_V) s_val[pos] = v[j];
+					}
+				}
+			}
+		}
+		barrier();
+		moved = true;
+		if (p + 1 < passes) {
+#pragma unroll
+			for (int j = 0; j < R; ++j) {
+				const uint32_t i = local + j * 16;
+				if ((uint32_t)j < rounds && i < held) {
+					k[j] = s_key[i];
+					if constexpr (HAS_V) v[j] = s_val[i];
+				}
+			}
+		}
+	}
+	if (moved) {
+		for (uint32_t i = tid; i < held; i += kClThreads) {
+			kout[first + i] = s_key[i];
+			if constexpr (HAS_V) vout[first + i] = s_val[i];
+		}
+	} else {
+#pragma unroll
+		for (int j = 0; j < R; ++j) {
+			const uint32_t i = local + j * 16;
+			if ((uint32_t)j < rounds && i < held) {
+				kout[first + i] = k[j];
+				if constexpr (HAS_V) vout[first + i] = v[j];
+			}
+		}
+	}
+	// No CTA leaves while another may still read its totals.
+	if constexpr (CL > 1) barrier();
+}
+
 // Tile shape of the pass by the 32-bit register words a key (and value)
 // takes: keys per thread and resident CTAs per SM, each the measured best
 // at 2^27 - 2^28 elements (larger tiles spread the per-tile work -- row
@@ -842,6 +1072,54 @@ cudaError_t sort_tiles(const K *src, K *dst, V *vals, size_t n, int passes,
 	return e;
 }
 
+// One-byte keys without values: their sorted order is their histogram.
+inline cudaError_t sort_bytes(const uint8_t *src, uint8_t *dst, size_t n, CCLContext *ctx,
+	cudaStream_t s, GError **err) {
+	char *tmp = (char *)tmp_alloc(ctx, control_words(1) * 4, s, err);
+	if (!tmp) return cudaErrorMemoryAllocation;
+	UpTail tail = {};
+	tail.c = control_at((uint32_t *)tmp, 1);
+	tail.n = n;
+	cudaError_t e;
+	{
+		KernelTimer t("satradix_upsweep", s, (double)n);
+		e = launch_upsweep<uint8_t>(1, s, src, n, ctx->sm_count, tail);
+		t.stop();
+	}
+	if (e == cudaSuccess) {
+		const size_t vecs = (n + 15) / 16;
+		const unsigned grid = (unsigned)std::min<size_t>((vecs + kFillBytesThreads - 1) /
+			kFillBytesThreads, 8 * (size_t)ctx->sm_count);
+		KernelTimer t("satradix_fill", s, (double)n);
+		e = launch_chained(radix_fill_bytes, grid, kFillBytesThreads, 0, s, 1, dst, n,
+			(const uint32_t *)tail.c.base);
+		t.stop();
+	}
+	count_launches(3);
+	tmp_free(tmp, s);
+	if (e != cudaSuccess) cuda_ok(e, err, "satradix");
+	return e;
+}
+
+template <typename K, typename V, bool HAS_V, int CL>
+cudaError_t sort_cluster(const K *src, K *dst, V *vals, size_t n, int passes, cudaStream_t s,
+	GError **err) {
+	const size_t rounds = (n + (size_t)CL * kClThreads - 1) / ((size_t)CL * kClThreads);
+	const size_t smem = cluster_smem<K, V, HAS_V>(rounds * kClThreads);
+	auto kern = radix_cluster<K, V, HAS_V, CL>;
+	cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+		(int)cluster_smem<K, V, HAS_V>(kClThreads * kClRounds));
+	if (e == cudaSuccess) {
+		KernelTimer t("satradix_cluster", s, 2.0 * (double)n * (sizeof(K) + (HAS_V ? sizeof(V) : 0)));
+		e = launch_chained(kern, CL, kClThreads, smem, s, CL, src, dst, (const V *)vals, vals,
+			(uint32_t)n, (uint32_t)rounds, passes);
+		t.stop();
+		count_launches(1);
+	}
+	if (e != cudaSuccess) cuda_ok(e, err, "satradix");
+	return e;
+}
+
 template <typename K, typename V, bool HAS_V>
 cudaError_t sort_typed(const void *src, void *dst, void *vals, size_t n, int sort_bits,
 	CCLContext *ctx, cudaStream_t s, GError **err) {
@@ -854,6 +1132,12 @@ cudaError_t sort_typed(const void *src, void *dst, void *vals, size_t n, int sor
 	const K *ks = (const K *)src;
 	K *kd = (K *)dst;
 	V *v = (V *)vals;
+	if (n <= kOneCtaKeys<K>) return sort_cluster<K, V, HAS_V, 1>(ks, kd, v, n, passes, s, err);
+	if constexpr (kClusterKeys<K, HAS_V> > 0) {
+		if (n <= kClusterKeys<K, HAS_V>)
+			return sort_cluster<K, V, HAS_V, 8>(ks, kd, v, n, passes, s, err);
+	}
+	if constexpr (sizeof(K) == 1 && !HAS_V) return sort_bytes(ks, kd, n, ctx, s, err);
 	// The smallest tile that leaves at most one tile per SM; beyond, large
 	// tiles.
 	const size_t sms = (size_t)ctx->sm_count;
