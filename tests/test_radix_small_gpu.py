@@ -66,3 +66,28 @@ def test_bytes(clops, ctx, queue, code, dt, n, kind, offset):
     clops.lib.ccl_buffer_destroy(w)
     b.destroy()
     s.destroy()
+
+
+@pytest.mark.parametrize("code,dt", [(3, np.uint16), (2, np.int16)])
+@pytest.mark.parametrize("n", [(5 << 18) - 1, 5 << 18, (5 << 18) + 77, 5 * (1 << 20) + 3])
+@pytest.mark.parametrize("kind", ["uniform", "one", "ends", "mostly_one", "spread"])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_two_byte_keys(clops, ctx, queue, code, dt, n, kind, offset):
+    """From 5 x 2^18 two-byte keys the output comes from the 65536-bin histogram:
+    counters that pass 2^15 and 2^16 in one CTA, runs of empty bins, bins of
+    one key."""
+    r = splitmix64(n, n) >> np.uint64(48)
+    a = {"uniform": r, "one": np.full(n, 0xFFFF), "ends": np.where(r < 40000, 0, 0xFFFF),
+         "mostly_one": np.where(np.arange(n) < 65536, np.arange(n), 513),
+         "spread": np.arange(n) % 65536}[kind].astype(np.uint16)
+    s = clops.Sorter(ctx, "satradix", code)
+    b = clops.Buffer(ctx, 2 * (n + offset + 1))
+    b.write(queue, np.concatenate([np.full(offset, 9), a, [9]]).astype(np.uint16))
+    w = clops.call(clops.lib.ccl_buffer_new_wrap, ctx.h, b.ptr + 2 * offset, 2 * n)
+    clops.wait(clops.call(clops.lib.clo_sort_with_device_data, s.h, queue.h, None, w, None, n, 0))
+    got = b.read(queue, np.uint16, n + offset + 1)
+    np.testing.assert_array_equal(got[offset:-1], np.sort(a))
+    assert got[-1] == 9 and np.all(got[:offset] == 9)
+    clops.lib.ccl_buffer_destroy(w)
+    b.destroy()
+    s.destroy()
