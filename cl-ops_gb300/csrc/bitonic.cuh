@@ -195,8 +195,7 @@ bitonic_global_steps_v(T *data, size_t groups, int stage, int step) {
 }
 
 // ------------------------------------------------------- register tiles
-// A thread holds 2^RE elements (128 bytes of 4- and 8-byte types) in
-// registers. In layout L(B) register m of thread g (its id within the tile:
+// A thread holds 2^RE elements in registers. In layout L(B) register m of thread g (its id within the tile:
 // cluster rank above the thread index) holds tile element
 //   ((g >> B) << (B + RE)) | (m << B) | (g & (2^B - 1)),
 // so the steps on index bits B .. B + RE - 1 are compare-exchanges between
@@ -210,31 +209,28 @@ bitonic_global_steps_v(T *data, size_t groups, int stage, int step) {
 // its 2^K consecutive elements. The phase on the cluster's bits takes the
 // layout L(T - RE), whose registers span the CTAs: it is entered by reading
 // the other CTAs' shared memory and left by writing into it (or entered
-// straight from global memory, in a finish). A tile of 2^15 elements over 8
-// SMs sorts in about a third of the time one SM takes for 2^14, and the
-// stages between K and T need no global passes of their own.
+// straight from global memory, in a finish). 2^15 4-byte elements sort in one
+// launch on 8 SMs in about a third of the time one SM takes for 2^14.
 //
 // No barrier is needed before a transpose's writes: a thread writes exactly
 // the slots it read itself in the transpose before (each slot has one owner
 // per layout). After them the barrier covers the threads that read them:
 // the warp for layouts up to L(5) (a warp holds the same 2^(RE+5)
 // consecutive elements in each of them), the CTA, or the cluster.
-template <typename T>
-constexpr int kRE = sizeof(T) == 8 ? 4 : 5;
-
-template <typename T, int K, int LOGC>
+template <typename T, int K_, int LOGC_, int RE_>
 struct TileCfg {
-	static constexpr int RE = kRE<T>, R = 1 << RE, TL = K + LOGC;
-	static constexpr int kK = K, kThreads = 1 << (K - RE), kCluster = 1 << LOGC;
+	static constexpr int kK = K_, LOGC = LOGC_, RE = RE_, R = 1 << RE, TL = kK + LOGC;
+	static constexpr int kThreads = 1 << (kK - RE), kCluster = 1 << LOGC;
 	static constexpr int LR = TL - RE;  // the cluster phase's layout
-	static constexpr size_t kSmem = ((size_t)(1 << K) + (1 << (K - RE))) * sizeof(T);
-	static constexpr int kMinBlocks = (sizeof(T) == 8 ? 768 : 1024) / kThreads;
+	static constexpr size_t kSmem = ((size_t)(1 << kK) + (1 << (kK - RE))) * sizeof(T);
+	// (64 registers a thread, 80 with 16 8-byte elements.)
+	static constexpr int kMinBlocks = (sizeof(T) == 8 && RE == 4 ? 768 : 1024) / kThreads;
 };
 
-template <typename T, int K, int LOGC>
+template <typename T, typename CFG>
 struct RegTile {
-	using C = TileCfg<T, K, LOGC>;
-	static constexpr int RE = C::RE, R = C::R, TL = C::TL;
+	using C = CFG;
+	static constexpr int RE = C::RE, R = C::R, TL = C::TL, K = C::kK, LOGC = C::LOGC;
 	T r[R];
 	T *s;
 	uint32_t tid, rank, g;
@@ -384,14 +380,14 @@ struct RegTile {
 	}
 };
 
-// A CTA's 2^K elements between global memory and L(0). A thread's 128
-// consecutive bytes move as 32-byte vectors when the part is 32-byte aligned
-// (half the requests of 16-byte vectors, whose lanes 128 bytes apart each
+// A CTA's 2^K elements between global memory and L(0). A thread's
+// consecutive elements move as 32-byte vectors when the part is 32-byte aligned
+// (half the requests of 16-byte vectors, whose lanes 64 or 128 bytes apart each
 // touch a line of their own) and wholly valid, else coalesced element by
 // element through a transpose, elements from `valid` on reading as the pad.
 template <typename Tile, typename T>
 __device__ __forceinline__ void tile_load(Tile &t, const T *p, size_t valid, T pad) {
-	constexpr int K = Tile::C::kK, B = K - Tile::RE, R = Tile::R;
+	constexpr int K = Tile::K, B = K - Tile::RE, R = Tile::R;
 	if (sizeof(T) >= 4 && valid >= ((size_t)1 << K) && ((uintptr_t)p % 32) == 0) {
 		const char *src = reinterpret_cast<const char *>(p) + (size_t)t.tid * (R * sizeof(T));
 		uint32_t w[R * sizeof(T) / 4 + 1];
@@ -417,7 +413,7 @@ __device__ __forceinline__ void tile_load(Tile &t, const T *p, size_t valid, T p
 
 template <typename Tile, typename T>
 __device__ __forceinline__ void tile_store(Tile &t, T *p, size_t valid) {
-	constexpr int K = Tile::C::kK, B = K - Tile::RE, R = Tile::R;
+	constexpr int K = Tile::K, B = K - Tile::RE, R = Tile::R;
 	if (sizeof(T) >= 4 && valid >= ((size_t)1 << K) && ((uintptr_t)p % 32) == 0) {
 		char *dst = reinterpret_cast<char *>(p) + (size_t)t.tid * (R * sizeof(T));
 		uint32_t w[R * sizeof(T) / 4 + 1];
@@ -448,15 +444,15 @@ __device__ __forceinline__ void tile_store(Tile &t, T *p, size_t valid) {
 // n_src on are the pad) into `dst`. Otherwise: steps T .. 1 of `stage` (> T)
 // of every tile of `src` into `dst` (the same array, or in the last stage
 // the caller's). Elements of `dst` from n_dst on are not written.
-template <typename T, int K, int LOGC, bool SORT>
-__global__ void __launch_bounds__((TileCfg<T, K, LOGC>::kThreads), (TileCfg<T, K, LOGC>::kMinBlocks))
+template <typename T, typename C, bool SORT>
+__global__ void __launch_bounds__(C::kThreads, C::kMinBlocks)
 bitonic_tile(const T *src, T *dst, size_t n_src, size_t n_dst, int stage) {
-	using C = TileCfg<T, K, LOGC>;
+	constexpr int K = C::kK, LOGC = C::LOGC;
 	// Doubles travel as their bits (see ord).
 	constexpr bool kOrd = std::is_same<T, double>::value;
 	using U = typename std::conditional<kOrd, int64_t, T>::type;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
-	RegTile<U, K, LOGC> t;
+	RegTile<U, C> t;
 	t.s = reinterpret_cast<U *>(smem_raw);
 	t.tid = threadIdx.x;
 	t.rank = LOGC ? dev::cluster_rank() : 0u;
@@ -524,7 +520,7 @@ bitonic_tile(const T *src, T *dst, size_t n_src, size_t n_dst, int stage) {
 #pragma unroll
 			for (int m = 0; m < C::R; ++m) t.r[m] = ord(t.r[m]);
 		} else {
-			RegTile<T, K, LOGC> f;
+			RegTile<T, C> f;
 			f.s = reinterpret_cast<T *>(smem_raw);
 			f.tid = t.tid;
 			f.rank = t.rank;
@@ -680,14 +676,14 @@ constexpr int kGlobalSteps = sizeof(T) == 4 ? 7 : sizeof(T) == 1 ? 5 : 6;
 
 // The sort with one tile configuration. `work` holds N elements (it may be
 // `dst` when n == N; null when one tile holds everything).
-template <typename T, int K, int LOGC>
+template <typename T, typename C>
 cudaError_t run_tiles(const T *src, T *dst, T *work, size_t n, int logN, cudaStream_t s,
 	unsigned &launches) {
-	using C = TileCfg<T, K, LOGC>;
+	constexpr int K = C::kK;
 	const size_t N = (size_t)1 << logN;
 	const int TL = C::TL;
-	auto sort_k = bitonic_tile<T, K, LOGC, true>;
-	auto fin_k = bitonic_tile<T, K, LOGC, false>;
+	auto sort_k = bitonic_tile<T, C, true>;
+	auto fin_k = bitonic_tile<T, C, false>;
 	cudaError_t e = cudaSuccess;
 	if (C::kSmem > 48 * 1024) {
 		e = cudaFuncSetAttribute(sort_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::kSmem);
@@ -751,16 +747,26 @@ cudaError_t run_rounds(T *d, int logN, int max_ps, int max_sfs, cudaStream_t s,
 	return e;
 }
 
-// Tile configurations by size: one CTA of 2^12 elements; clusters of eight of
-// those up to 2^kClusterMax elements, where tiles of one CTA would leave most
-// SMs idle; then tiles of one CTA of 2^14 (2^13 of 8 bytes), whose passes
-// move more bytes a second. Measured (us a sort, clusters / one CTA), int:
-// 2^19 46.5 / 61, 2^20 60 / 72, 2^21 103 / 88; double: 2^19 103 / 109, 2^20
-// 137 / 131. Parts of 2^13 and 2^14 elements per CTA and clusters of 2 and 4
-// were slower at every size.
-constexpr int kOneCta = 12;
+// Tiles by size and type. Up to kOneTile elements one tile does the whole
+// sort: one CTA of 2^kSmallK elements, or (types up to 4 bytes) a cluster of
+// eight of those. Beyond, tiles of one such CTA; small ones keep all SMs busy
+// and their launches, chained, are cheap. us a sort:
+//   float, tiles of 2^12 / 2^13 / 2^14 (16 elements a thread): 2^16 20.3 / 26.4
+//   / -, 2^20 55.3 / 54.9 / -, 1.5 x 10^6 78.2 / 89.3 / -, 2^24 596 / 635 / -;
+//   32 elements a thread: 2^16 22.7 / 27.3 / 41, 2^24 657 / 632 / 659; clusters
+//   of eight over 2^12: 2^16 26, 2^20 63, 2^24 755; 2^15 14.6 in one cluster
+//   against 17 in five launches.
+//   double, 2^11 by 8 / 2^13 by 16: 2^16 36 / 63, 2^20 138 / 132, 2^22 496 /
+//   500, 2^24 2358 / 2141; clusters of eight over 2^12 by 16: 2^16 44.
+//   char, 32 / 16 elements a thread: 2^16 27 / 26, 2^24 673 / 729.
 template <typename T>
-constexpr int kClusterMax = sizeof(T) == 8 ? 19 : 20;
+using SmallTile = typename std::conditional<sizeof(T) == 8, TileCfg<T, 11, 0, 3>,
+	TileCfg<T, 12, 0, sizeof(T) == 1 ? 5 : 4>>::type;
+template <typename T>
+using ClusterTile = TileCfg<T, 12, 3, sizeof(T) == 1 ? 5 : 4>;
+template <typename T>
+constexpr int kOneTile = sizeof(T) == 8 ? 11 : 15;
+constexpr int kBigDoubleMin = 23;  // log2: 8-byte tiles of 2^13 from here
 
 template <typename T>
 cudaError_t sort_typed(const T *src, T *dst, size_t n, int max_ps, int max_sfs,
@@ -772,7 +778,7 @@ cudaError_t sort_typed(const T *src, T *dst, size_t n, int max_ps, int max_sfs,
 	T *tmp = nullptr;
 	const int t0 = std::min(sizeof(T) >= 8 ? 13 : 14, logN);
 	const bool rounds = max_ps < 4 || (max_sfs >= 1 && max_sfs < t0);
-	if (N != n && (rounds || logN > kOneCta + 3)) {
+	if (N != n && (rounds || logN > kOneTile<T>)) {
 		tmp = (T *)tmp_alloc(ctx, N * sizeof(T), s, err);
 		if (!tmp) return cudaErrorMemoryAllocation;
 	}
@@ -790,12 +796,16 @@ cudaError_t sort_typed(const T *src, T *dst, size_t n, int max_ps, int max_sfs,
 		if (e == cudaSuccess) e = run_rounds<T>(work, logN, max_ps, max_sfs, s, launches);
 		if (e == cudaSuccess && tmp)
 			e = cudaMemcpyAsync(dst, tmp, n * sizeof(T), cudaMemcpyDeviceToDevice, s);
-	} else if (logN <= kOneCta) {
-		e = run_tiles<T, kOneCta, 0>(src, dst, work, n, logN, s, launches);
-	} else if (logN <= kClusterMax<T>) {
-		e = run_tiles<T, kOneCta, 3>(src, dst, work, n, logN, s, launches);
+	} else if (logN > SmallTile<T>::kK && logN <= kOneTile<T>) {
+		if constexpr (sizeof(T) <= 4)
+			e = run_tiles<T, ClusterTile<T>>(src, dst, work, n, logN, s, launches);
 	} else {
-		e = run_tiles<T, sizeof(T) == 8 ? 13 : 14, 0>(src, dst, work, n, logN, s, launches);
+		bool big = false;
+		if constexpr (sizeof(T) == 8) {
+			big = logN >= kBigDoubleMin;
+			if (big) e = run_tiles<T, TileCfg<T, 13, 0, 4>>(src, dst, work, n, logN, s, launches);
+		}
+		if (!big) e = run_tiles<T, SmallTile<T>>(src, dst, work, n, logN, s, launches);
 	}
 	if (tmp) tmp_free(tmp, s);
 	count_launches(launches);
