@@ -37,11 +37,13 @@ cudaError_t radix_sort(const void *src, void *dst, void *vals, size_t n, int key
 	}
 	if (none) return cudaSuccess;
 	// Small whole-key sorts without values: equal keys are the same bits, so
-	// any sort gives the stable one's result, and the bitonic tile kernel does
-	// up to 2^15 elements in one launch and no scratch (us, bitonic / the radix
-	// sort's best: 2^10 u32 5.1 / 8.2, 2^12 6.5 / 11, 2^15 15 / 25, 2^10 u64 9.9
-	// / 15, 2^15 33 / 44; keys of one and two bytes are faster by radix).
-	if (val_bytes == 0 && key_bytes >= 4 && sort_bits == 8 * key_bytes && n <= ((size_t)1 << 15))
+	// any sort gives the stable one's result, and the bitonic tiles are faster
+	// while launches and latencies, not bytes, are what a sort costs (us,
+	// bitonic / the radix sort's best: u32 2^10 4.4 / 8.2, 2^15 14 / 25, 2^17 24
+	// / 27.5, 2^18 30 / 28; u64 2^10 6.2 / 15, 2^15 22 / 44, 2^18 41 / 58, 2^20
+	// 101 / 80; keys of one and two bytes are faster by radix).
+	if (val_bytes == 0 && key_bytes >= 4 && sort_bits == 8 * key_bytes &&
+		n <= ((size_t)1 << (key_bytes == 8 ? 18 : 17)))
 		return bitonic_sort(src, dst, n, key_bytes == 8 ? CLO_ULONG : CLO_UINT, 4, 0, ctx, s, err);
 	switch (key_bytes) {
 	case 1: return radix::sort<uint8_t>(src, dst, vals, n, val_bytes, sort_bits, ctx, s, err);

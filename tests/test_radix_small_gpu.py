@@ -91,3 +91,18 @@ def test_two_byte_keys(clops, ctx, queue, code, dt, n, kind, offset):
     clops.lib.ccl_buffer_destroy(w)
     b.destroy()
     s.destroy()
+
+
+@pytest.mark.parametrize("code,dt,n", [(5, np.uint32, 50000), (5, np.uint32, 1 << 17),
+                                       (4, np.int32, (1 << 17) + 1), (7, np.uint64, (1 << 18) - 3),
+                                       (7, np.uint64, (1 << 18) + 1)])
+def test_whole_keys_around_the_bitonic_limit(clops, ctx, queue, code, dt, n):
+    a = keys_of_type(n, n, dt)
+    s = clops.Sorter(ctx, "satradix", code)
+    bi = clops.Buffer.from_array(ctx, queue, a)
+    bo = clops.Buffer(ctx, a.nbytes)
+    clops.wait(s.sort_device(queue, bi, n, buf_out=bo))
+    np.testing.assert_array_equal(bo.read(queue, dt, n), oracle.radix_sort(a))
+    np.testing.assert_array_equal(bi.read(queue, dt, n), a)
+    for x in (bi, bo, s):
+        x.destroy()
