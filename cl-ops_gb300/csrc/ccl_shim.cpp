@@ -440,9 +440,20 @@ CCLEvent *ccl_buffer_enqueue_copy(CCLBuffer *src_buf, CCLBuffer *dst_buf,
 		return nullptr;
 	if (!clo::wait_ewl(cq, evt_wait_lst, err)) return nullptr;
 	ccl_event *e = clo::event_begin(cq, "copy");
-	if (!cuda_ok(cudaMemcpyAsync((char *)dst_buf->ptr + dst_offset,
-			(char *)src_buf->ptr + src_offset, size, cudaMemcpyDeviceToDevice,
-			cq->stream), err, "enqueue_copy"))
+	// A small copy within the queue's device (the current one: a kernel needs
+	// that) is a chained kernel, so that the kernels after it chain on (a sort
+	// of 1000 pairs with two copies: 16.4 us with memory copies, 11.2 so).
+	char *dst = (char *)dst_buf->ptr + dst_offset;
+	const char *src = (const char *)src_buf->ptr + src_offset;
+	const int on = cq->ctx->ordinal;
+	int current = -1;
+	const bool small = size > 0 && size <= clo::kCopyChainedMax &&
+		cudaGetDevice(&current) == cudaSuccess && current == on &&
+		src_buf->ctx->ordinal == on && dst_buf->ctx->ordinal == on &&
+		(((uintptr_t)dst | (uintptr_t)src) % 16) == 0 && (dst >= src + size || src >= dst + size);
+	if (!cuda_ok(small ? clo::copy_chained(dst, src, size, cq->stream)
+					   : cudaMemcpyAsync(dst, src, size, cudaMemcpyDeviceToDevice, cq->stream),
+			err, "enqueue_copy"))
 		return nullptr;
 	clo::event_end(e);
 	return e;

@@ -138,6 +138,11 @@ cudaError_t radix_msd_partition(const void *keys_in, void *keys_out, size_t n, i
 // the chaining.
 cudaError_t clear_chained(void *p, size_t bytes, cudaStream_t s);
 
+// A device-to-device copy as a chained kernel, for copies too small for their
+// time to be the bytes (kCopyChainedMax); the ranges must not overlap.
+constexpr size_t kCopyChainedMax = (size_t)4 << 20;
+cudaError_t copy_chained(void *dst, const void *src, size_t bytes, cudaStream_t s);
+
 // Exclusive scan: out[i] = sum_{j<i} (sum type) in[j] modulo
 // 2^(8*out_bytes). in_type is an integer CloType, out_bytes in {1,2,4,8}.
 cudaError_t scan_exclusive(const void *in, void *out, size_t n,

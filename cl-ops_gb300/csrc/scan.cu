@@ -259,6 +259,17 @@ __global__ void __launch_bounds__(256) clear_words(uint4 *words, size_t count) {
 		words[i] = make_uint4(0, 0, 0, 0);
 }
 
+// 16-byte vectors where both addresses allow them (tail and otherwise bytes).
+__global__ void __launch_bounds__(256) copy_words(char *dst, const char *src, size_t bytes) {
+	dev::pdl_wait();
+	const size_t vecs = (((uintptr_t)dst | (uintptr_t)src) % 16) == 0 ? bytes / 16 : 0;
+	const size_t first = blockIdx.x * (size_t)256 + threadIdx.x, stride = (size_t)gridDim.x * 256;
+#pragma unroll 4
+	for (size_t i = first; i < vecs; i += stride)
+		reinterpret_cast<uint4 *>(dst)[i] = reinterpret_cast<const uint4 *>(src)[i];
+	for (size_t i = vecs * 16 + first; i < bytes; i += stride) dst[i] = src[i];
+}
+
 // Per device and type pair, once: records the kernel's resident CTAs per SM.
 // Later calls (possibly while a graph is being captured) only read
 // the cached count.
@@ -371,6 +382,12 @@ cudaError_t clear_chained(void *p, size_t bytes, cudaStream_t s) {
 	count_launches(1);
 	return launch_chained(clear_words, (unsigned)std::min<size_t>((vecs + 1023) / 1024, 608), 256, 0,
 		s, 1, (uint4 *)p, vecs);
+}
+
+cudaError_t copy_chained(void *dst, const void *src, size_t bytes, cudaStream_t s) {
+	count_launches(1);
+	return launch_chained(copy_words, (unsigned)std::min<size_t>((bytes + 4095) / 4096, 608), 256, 0,
+		s, 1, (char *)dst, (const char *)src, bytes);
 }
 
 // Tile whose publication is withheld (-1: none). Only the watchdog test
