@@ -508,8 +508,8 @@ __global__ void __launch_bounds__(256) seg_heads(const uint64_t *off, uint32_t S
 // Segmented exclusive scan: out[i] = sum of in[j] for j from the start of
 // i's segment to i - 1, for i in [off[0], off[S]); nothing else is written.
 // The combine of (head seen, sum) pairs is the usual segmented one: a
-// later head discards what came before it. Same tile layout and pipeline
-// as the plain scan (csrc/scan_tile.cuh): persistent CTAs take 8192-element
+// later head discards what came before it. The plain scan's pipeline on
+// tiles staged in shared memory (csrc/scan_tile.cuh): persistent CTAs take 8192-element
 // tiles in order; while warp 0 looks back, every warp prefetches the next
 // tile and its 32 head words, finds its last head (max-reduction) and sums
 // the elements from there on, so the next tile's (head seen, sum) is
