@@ -15,7 +15,7 @@
 // inclusive prefix. Status words carry their own ready bits, so neither side
 // needs a memory fence. Every wait is bounded. Staging the tile in shared
 // memory (a lane scanning 16 consecutive elements, seven shared wavefronts
-// per 32 elements for uint -> ulong) took 589 us at 2^28 against 551.
+// per 32 elements for uint -> ulong) took 589 us at 2^28 against 519.
 //
 // HBM roofline: sizeof(in) + sizeof(out) bytes per element (12 B for
 // uint -> ulong), plus 32 B of tile status per tile.
@@ -57,9 +57,10 @@ __device__ __forceinline__ Acc shfl_up(Acc v, int d) {
 // launched one; after the outputs the prefetched tile becomes the current
 // one. Every wait is on a lower tile id (down to tile 0, which
 // publishes its prefix at once), so the waits cannot form a cycle.
-template <typename InT, typename OutT, int THREADS, int TILE, int MINB>
+template <typename InT, typename OutT, int THREADS, int TILE, int MINB, bool KEEP = false>
 struct ScanCfg {
 	static constexpr int kThreads = THREADS, kTile = TILE, kMinBlocks = MINB;
+	static constexpr bool kKeepShared = KEEP;
 	using R = Rows<InT, OutT, THREADS, TILE>;
 };
 // Sums of one or two bytes, or narrower than the input: one shape for all.
@@ -69,16 +70,27 @@ template <bool C, typename A, typename B>
 using If = typename std::conditional<C, A, B>::type;
 
 // Threads, tile and resident CTAs per SM (registers: 65536 / (CTAs x
-// threads); the current and the prefetched tile take most of them). The tile
-// rate is bounded by the lookback (a window of 64 tiles a round trip, about
-// 80 tiles a microsecond), so narrow types take tiles twice as long. Measured
-// at 2^28 (us, 8192-element tiles at the same registers / these): uint ->
-// uint 406 / 375, uchar -> uint 404 / 255. uint -> ulong: 8192 551, 16384 at
-// one CTA 590, 512 threads 592. Windows of 96 and 128 tiles: 600 and 634.
+// threads)), and whether the current tile waits in shared memory while the
+// next one is loaded (KEEP: each thread parks its own vectors, conflict-free;
+// the two tiles' registers otherwise leave one CTA fewer an SM, or spills).
+// The tile rate is bounded by the lookback (a window of 64 tiles a round trip,
+// about 80 tiles a microsecond), so narrow types take tiles twice as long.
+// Measured at 2^28 (us): uint -> ulong two CTAs 559, three with KEEP 519, four
+// 547; ulong -> ulong 804 / 694 (two CTAs) / 1023 (three); uint -> uint
+// 16384-element tiles 380 / 356 (two) / 498 (three), 8192 406; uchar -> uint
+// 16384 255 (three), 8192 404. Windows of 96 and 128 tiles
+// and 512-thread CTAs were slower.
 template <typename InT, typename OutT>
 using ScanBig = If<kOneShape<InT, OutT>, ScanCfg<InT, OutT, 256, 8192, 1>,
-	If<sizeof(OutT) == 8, ScanCfg<InT, OutT, 256, 8192, 2>,
-	If<sizeof(InT) == 4, ScanCfg<InT, OutT, 256, 16384, 2>, ScanCfg<InT, OutT, 256, 16384, 3>>>>;
+	If<sizeof(OutT) == 8, If<sizeof(InT) == 8, ScanCfg<InT, OutT, 256, 8192, 2, true>,
+		If<sizeof(InT) == 4, ScanCfg<InT, OutT, 256, 8192, 3, true>, ScanCfg<InT, OutT, 256, 8192, 2>>>,
+	If<sizeof(InT) == 4, ScanCfg<InT, OutT, 256, 16384, 2, true>, ScanCfg<InT, OutT, 256, 16384, 3>>>>;
+// From kSmallMax to kMidMax elements uint -> ulong tiles stay in registers: with
+// about one tile a CTA nothing is prefetched (2^22 16.2 us against 17.9).
+constexpr size_t kMidMax = (size_t)1 << 23;
+template <typename InT, typename OutT>
+using ScanMid = If<sizeof(InT) == 4 && sizeof(OutT) == 8, ScanCfg<InT, OutT, 256, 8192, 2>,
+	ScanBig<InT, OutT>>;
 // Up to kSmallMax elements, 4096-element tiles: twice the CTAs, each with
 // half the rows to scan (2^18 uint -> ulong 6.3 us against 8.0, 2^20 8.3
 // against 9.1; 2^22 20.8 against 17.5).
@@ -105,6 +117,9 @@ scan_lookback(const InT *in, OutT *out, size_t n, TileStatus ts,
 	__shared__ Acc s_next_tot[kWarps];
 	__shared__ Acc s_excl;
 	__shared__ uint32_t s_tile, s_next;
+	static_assert(!CFG::kKeepShared || R::kWords % 4 == 0, "parked in 16-byte vectors");
+	constexpr int KR = CFG::kKeepShared ? R::kRows * R::kWords / 4 : 1;
+	extern __shared__ uint4 s_cur[];  // [KR][kThreads] with KEEP
 
 	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 	const uint32_t num_tiles = (uint32_t)((n + kTile - 1) / kTile);
@@ -153,6 +168,13 @@ scan_lookback(const InT *in, OutT *out, size_t n, TileStatus ts,
 		for (int r = 0; r < kRows; ++r) {
 			ex[r] = inc[r] - ex[r] + wsum;
 			wsum += __shfl_sync(0xffffffffu, inc[r], 31);
+		}
+		// The tile waits here while the next one takes the registers.
+		if constexpr (CFG::kKeepShared) {
+			const uint32_t *w = &cur.w[0][0];
+#pragma unroll
+			for (int i = 0; i < KR; ++i)
+				s_cur[i * CFG::kThreads + tid] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
 		}
 		if (lane == 0) s_warp_tot[warp] = wsum;
 		__syncthreads();
@@ -222,6 +244,18 @@ scan_lookback(const InT *in, OutT *out, size_t n, TileStatus ts,
 		const bool full = full_seg(seg);
 #pragma unroll
 		for (int r = 0; r < kRows; ++r) {
+			if constexpr (CFG::kKeepShared) {
+#pragma unroll
+				for (int i = 0; i < R::kWords / 4; ++i) {
+					uint32_t a, b, c, d;
+					asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(a), "=r"(b), "=r"(c), "=r"(d)
+						: "r"(dev::smem_u32(&s_cur[(r * R::kWords / 4 + i) * CFG::kThreads + tid])) : "memory");
+					cur.w[r][4 * i] = a;
+					cur.w[r][4 * i + 1] = b;
+					cur.w[r][4 * i + 2] = c;
+					cur.w[r][4 * i + 3] = d;
+				}
+			}
 			Acc run = base + ex[r];
 			const size_t i0 = seg + (size_t)(32 * r + lane) * kE;
 			if (full) {
@@ -270,6 +304,11 @@ __global__ void __launch_bounds__(256) copy_words(char *dst, const char *src, si
 	for (size_t i = vecs * 16 + first; i < bytes; i += stride) dst[i] = src[i];
 }
 
+template <typename CFG>
+constexpr size_t scan_shared() {
+	return CFG::kKeepShared ? (size_t)CFG::kThreads * CFG::R::kRows * CFG::R::kWords * 4 : 0;
+}
+
 // Per device and type pair, once: records the kernel's resident CTAs per SM.
 // Later calls (possibly while a graph is being captured) only read
 // the cached count.
@@ -286,8 +325,12 @@ cudaError_t scan_prepare(int *per_sm) {
 		std::lock_guard<std::mutex> lk(mu);
 		v = cached[dev].load(std::memory_order_relaxed);
 		if (v == 0) {
-			e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, scan_lookback<InT, OutT, CFG>,
-				CFG::kThreads, 0);
+			if (scan_shared<CFG>() > 48 * 1024)
+				e = cudaFuncSetAttribute(scan_lookback<InT, OutT, CFG>,
+					cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scan_shared<CFG>());
+			if (e == cudaSuccess)
+				e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, scan_lookback<InT, OutT, CFG>,
+				CFG::kThreads, scan_shared<CFG>());
 			if (e != cudaSuccess) return e;
 			if (v < 1) v = 1;
 			cached[dev].store(v, std::memory_order_release);
@@ -339,7 +382,7 @@ cudaError_t launch_scan_cfg(const void *in, void *out, size_t n, CCLContext *ctx
 	if (e == cudaSuccess) {
 		KernelTimer t("scan_lookback", s, (double)n * (sizeof(InT) + sizeof(OutT)));
 		e = launch_chained(scan_lookback<InT, OutT, CFG>, scan_grid(tiles, per_sm, ctx->sm_count),
-			CFG::kThreads, 0, s, 1, (const InT *)in, (OutT *)out, n, ts, ctx->d_status,
+			CFG::kThreads, scan_shared<CFG>(), s, 1, (const InT *)in, (OutT *)out, n, ts, ctx->d_status,
 			scan_vec(in, out), debug_skip_tile, carry_in, carry_out);
 		t.stop();
 		count_launches(1);
@@ -358,6 +401,7 @@ cudaError_t launch_scan(const void *in, void *out, size_t n, CCLContext *ctx,
 	};
 	if (n <= ScanOne<InT, OutT>::kTile) return go(ScanOne<InT, OutT>());
 	if (n <= kSmallMax) return go(ScanSmall<InT, OutT>());
+	if (n <= kMidMax) return go(ScanMid<InT, OutT>());
 	return go(ScanBig<InT, OutT>());
 }
 
@@ -545,7 +589,7 @@ cudaError_t launch_scan_noalloc(const void *in, void *out, size_t n,
 	int per_sm = 1;
 	e = scan_prepare<InT, OutT, CFG>(&per_sm);
 	if (e != cudaSuccess) return e;
-	scan_lookback<InT, OutT, CFG><<<scan_grid(tiles, per_sm, sm_count), CFG::kThreads, 0,
+	scan_lookback<InT, OutT, CFG><<<scan_grid(tiles, per_sm, sm_count), CFG::kThreads, scan_shared<CFG>(),
 		s>>>((const InT *)in, (OutT *)out, n, ts, dev_status, scan_vec(in, out), -1, nullptr,
 		nullptr);
 	count_launches(1);
