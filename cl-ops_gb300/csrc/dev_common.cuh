@@ -156,6 +156,10 @@ __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
 		: "memory");
 	asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
+// Earlier plain shared-memory accesses before later bulk copies.
+__device__ __forceinline__ void fence_proxy_async() {
+	asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
 __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
 	asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
 		:: "r"(smem_u32(bar)), "r"(bytes) : "memory");

@@ -655,8 +655,10 @@ constexpr int kRowWords = kRadix + 8;
 __device__ __forceinline__ int row_of(int r) { return r * kRowWords + (r & 1) * 8; }
 
 // ------------------------------------------------------- onesweep pass
-// One tile per CTA, tiles claimed in order from an atomic counter, so every
-// tile a CTA waits on belongs to a CTA that is already running. Per tile:
+// Tiles are claimed in order from an atomic counter, one per CTA or, in large
+// sorts, one after the other by resident CTAs (the next one claimed once the
+// tile's status is out), so every tile a CTA waits on belongs to a CTA that is
+// running and waits on lower tiles only. Per tile:
 //  1. keys (and values) are loaded in half-warp units: unit u holds the
 //     tile's keys u * 16 KPT .. (u + 1) * 16 KPT - 1, round j of lane l the
 //     key 16 j + l, so a unit's (round, lane) order is index order;
@@ -727,7 +729,37 @@ constexpr size_t tiles_smem() {
 		sizeof(uint32_t) + (stage > land ? stage : land);
 }
 
-template <typename K, typename V, bool HAS_V, int THREADS, int KPT, int MINB, bool GROUPED>
+// How a pass takes its tiles: one a CTA, looking back by windows or by groups,
+// or tile after tile by resident CTAs.
+constexpr int kTilesOne = 0, kTilesGrouped = 1, kTilesLoop = 2;
+
+// n elements copied by the whole grid, eight 16-byte vectors a thread in
+// flight where both sides are aligned.
+template <typename T>
+__device__ __forceinline__ void copy_elements(const T *in, T *out, size_t n) {
+	const size_t threads = (size_t)gridDim.x * blockDim.x;
+	const size_t self = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+	size_t done = 0;
+	if ((((uintptr_t)in | (uintptr_t)out) & 15) == 0) {
+		const size_t vecs = n * sizeof(T) / 16;
+		const uint4 *a = reinterpret_cast<const uint4 *>(in);
+		uint4 *b = reinterpret_cast<uint4 *>(out);
+		constexpr int B = 8;
+		for (size_t i = self; i < vecs; i += B * threads) {
+			uint4 r[B];
+#pragma unroll
+			for (int j = 0; j < B; ++j)
+				if (i + j * threads < vecs) r[j] = a[i + j * threads];
+#pragma unroll
+			for (int j = 0; j < B; ++j)
+				if (i + j * threads < vecs) b[i + j * threads] = r[j];
+		}
+		done = vecs * (16 / sizeof(T));
+	}
+	for (size_t i = done + self; i < n; i += threads) out[i] = in[i];
+}
+
+template <typename K, typename V, bool HAS_V, int THREADS, int KPT, int MINB, int MODE>
 __global__ void __launch_bounds__(THREADS, MINB)
 radix_pass_tiles(const __grid_constant__ PassArgs<K, V> a, uint32_t num_tiles) {
 	constexpr int TILE = THREADS * KPT;
@@ -767,6 +799,17 @@ radix_pass_tiles(const __grid_constant__ PassArgs<K, V> a, uint32_t num_tiles) {
 	auto bulk_ok_for = [&](const K *k, const V *v) {
 		return BULK && ((uintptr_t)k % 16) == 0 && (!HAS_V || ((uintptr_t)v % 16) == 0);
 	};
+	// Tile tt's bulk copies (one thread).
+	auto issue = [&](const K *kin, const V *vin, uint32_t tt) {
+		dev::mbar_expect_tx(bar, (uint32_t)(TILE * (sizeof(K) + (HAS_V ? sizeof(V) : 0))));
+		const size_t t0 = (size_t)tt * TILE;
+#pragma unroll 1
+		for (int u = 0; u < UNITS; ++u) {
+			dev::bulk_g2s(land_k + u * LK, kin + t0 + u * UKEYS, (uint32_t)(UKEYS * sizeof(K)), bar);
+			if constexpr (HAS_V)
+				dev::bulk_g2s(land_v + u * LV, vin + t0 + u * UKEYS, (uint32_t)(UKEYS * sizeof(V)), bar);
+		}
+	};
 	if (owner) {
 #pragma unroll
 		for (int i = 0; i < HALF; ++i) s_cnt[row_of(i) + pd] = 0;
@@ -782,45 +825,49 @@ radix_pass_tiles(const __grid_constant__ PassArgs<K, V> a, uint32_t num_tiles) {
 		if ((plan & 3u) == kPlanRun && bulk_ok_for(kin, vin) && tt < num_tiles &&
 			(size_t)(tt + 1) * TILE <= a.n) {
 			dev::mbar_init(bar, 1);
-			dev::mbar_expect_tx(bar, (uint32_t)(TILE * (sizeof(K) + (HAS_V ? sizeof(V) : 0))));
-			const size_t t0 = (size_t)tt * TILE;
-#pragma unroll 1
-			for (int u = 0; u < UNITS; ++u) {
-				dev::bulk_g2s(land_k + u * LK, kin + t0 + u * UKEYS,
-					(uint32_t)(UKEYS * sizeof(K)), bar);
-				if constexpr (HAS_V)
-					dev::bulk_g2s(land_v + u * LV, vin + t0 + u * UKEYS,
-						(uint32_t)(UKEYS * sizeof(V)), bar);
-			}
+			issue(kin, vin, tt);
 		}
 	}
-	uint32_t gbase = owner ? a.base[pd] : 0;
+	const uint32_t gbase = owner ? a.base[pd] : 0;
 	__syncthreads();
-	const uint32_t t = s_misc[0], plan = s_misc[1];
-	if (t >= num_tiles || (plan & 3u) == kPlanSkip) return;
-	const K *__restrict__ kin = pick(a.keys, (plan >> 2) & 3u);
-	K *__restrict__ kout = pick(a.keys, (plan >> 4) & 3u);
-	const V *__restrict__ vin = pick(a.vals, (plan >> 2) & 3u);
-	V *__restrict__ vout = pick(a.vals, (plan >> 4) & 3u);
+	uint32_t t = s_misc[0];
+	// The plan's buffers: held where the registers allow it, else worked out
+	// where they are used (us a sort, held / not: u32 2^28 3163 / 3236, u64 2^27
+	// 4602 / 4566, (u32, u32) 2^27 2562 / 2466).
+	const uint32_t plan = s_misc[1];
+	const K *const kin0 = pick(a.keys, (plan >> 2) & 3u);
+	K *const kout0 = pick(a.keys, (plan >> 4) & 3u);
+	const V *const vin0 = pick(a.vals, (plan >> 2) & 3u);
+	V *const vout0 = pick(a.vals, (plan >> 4) & 3u);
+	uint32_t *const status0 = (plan >> 6) & 1u ? a.status[1] : a.status[0];
+	uint32_t *const status1 = (plan >> 6) & 1u ? a.status[0] : a.status[1];
+	if ((plan & 3u) == kPlanSkip) return;
 	if ((plan & 3u) == kPlanCopy) {
-		for (size_t i = (size_t)t * TILE + tid; i < a.n && i < (size_t)(t + 1) * TILE; i += THREADS) {
-			kout[i] = kin[i];
-			if constexpr (HAS_V) vout[i] = vin[i];
-		}
+		copy_elements(kin0, kout0, a.n);
+		if constexpr (HAS_V) copy_elements(vin0, vout0, a.n);
 		return;
 	}
-	uint32_t *status = (plan >> 6) & 1u ? a.status[1] : a.status[0];
-	uint32_t *status_next = (plan >> 6) & 1u ? a.status[0] : a.status[1];
-	const bool bulk_ok = bulk_ok_for(kin, vin);
+	constexpr bool HOLD = MODE != kTilesLoop || (sizeof(K) <= 4 && !HAS_V);
+	auto keys_in = [&] { return HOLD ? kin0 : pick(a.keys, (s_misc[1] >> 2) & 3u); };
+	auto keys_out = [&] { return HOLD ? kout0 : pick(a.keys, (s_misc[1] >> 4) & 3u); };
+	auto vals_in = [&] { return HOLD ? vin0 : pick(a.vals, (s_misc[1] >> 2) & 3u); };
+	auto vals_out = [&] { return HOLD ? vout0 : pick(a.vals, (s_misc[1] >> 4) & 3u); };
+	auto status_now = [&] { return HOLD ? status0 : (s_misc[1] >> 6) & 1u ? a.status[1] : a.status[0]; };
+	auto status_nxt = [&] { return HOLD ? status1 : (s_misc[1] >> 6) & 1u ? a.status[0] : a.status[1]; };
+	if (t >= num_tiles) return;
+	uint32_t parity = 0;
 
+	do {
 	// Keys (and values) of this thread's unit, round-major (index order).
 	K k[KPT];
 	V v[HAS_V ? KPT : 1];
+	const K *__restrict__ kin = keys_in();
+	const V *__restrict__ vin = vals_in();
 	const size_t ubase = (size_t)t * TILE + (size_t)unit * UKEYS;
-	if (bulk_ok && (size_t)(t + 1) * TILE <= a.n) {
-		if (!dev::mbar_wait_bounded(bar, 0)) {
+	if (bulk_ok_for(kin, vin) && (size_t)(t + 1) * TILE <= a.n) {
+		if (!dev::mbar_wait_bounded(bar, parity)) {
 			if (tid == 0) dev::report_timeout(a.dev_status, DEV_ERR_COPY_TIMEOUT, (int)t);
-			dev::mbar_wait_bounded(bar, 0);  // the copies still in flight
+			dev::mbar_wait_bounded(bar, parity);  // the copies still in flight
 		}
 #pragma unroll
 		for (int j = 0; j < KPT; ++j) {
@@ -841,8 +888,9 @@ radix_pass_tiles(const __grid_constant__ PassArgs<K, V> a, uint32_t num_tiles) {
 	// Unit prefixes of digit pd in unit order (written to the units' rank
 	// words, the tile offset added below) and the tile's count.
 	uint32_t sum = 0;
-	uint32_t *st = status + (size_t)t * kRadix + pd;
+	uint32_t *st = HOLD ? status0 + (size_t)t * kRadix + pd : nullptr;
 	if (owner) {
+		uint32_t *status = status_now(), *status_next = status_nxt();
 		uint32_t run = 0;
 #pragma unroll
 		for (int i = 0; i < HALF; ++i) {
@@ -856,9 +904,9 @@ radix_pass_tiles(const __grid_constant__ PassArgs<K, V> a, uint32_t num_tiles) {
 		}
 		sum = run;
 		// Publish the tile's count of digit pd (tile 0: its inclusive prefix).
-		dev::st_relaxed_u32(st, (t == 0 ? kStPrefix : kStAgg) | sum);
+		dev::st_relaxed_u32(HOLD ? st : status + (size_t)t * kRadix + pd, (t == 0 ? kStPrefix : kStAgg) | sum);
 		status_next[(size_t)t * kRadix + pd] = 0;
-		if constexpr (GROUPED) {
+		if constexpr (MODE == kTilesGrouped) {
 			const size_t g = ((size_t)num_tiles + t / kGroup) * kRadix + pd;
 			atomicAdd(status + g, kGroupOne + sum);
 			if (t % kGroup == 0) status_next[g] = 0;
@@ -900,7 +948,8 @@ radix_pass_tiles(const __grid_constant__ PassArgs<K, V> a, uint32_t num_tiles) {
 	// Lookback over the preceding tiles for digit pd (bounded waits).
 	uint32_t excl = 0;
 	if (owner && t > 0) {
-		if constexpr (GROUPED) {
+		uint32_t *status = status_now();
+		if constexpr (MODE == kTilesGrouped) {
 			excl = group_lookback(status, num_tiles, t, pd, a.dev_status);
 		} else {
 			long long base = (long long)t - 1;
@@ -919,11 +968,23 @@ radix_pass_tiles(const __grid_constant__ PassArgs<K, V> a, uint32_t num_tiles) {
 				}
 				done = lookback_window<kLookWindow>(status, pd, base, excl);
 			}
-			dev::st_relaxed_u32(st, kStPrefix | (excl + sum));
+			dev::st_relaxed_u32(HOLD ? st : status + (size_t)t * kRadix + pd, kStPrefix | (excl + sum));
 		}
 	}
 	if (owner) s_tile_off[pd] += excl;
 	__syncthreads();
+	// The next tile is claimed (its status comes after this tile's, which is
+	// out) and the counts cleared while the staged tile is written out.
+	uint32_t next = 0;
+	if constexpr (MODE == kTilesLoop) {
+		if (tid == 0) next = atomicAdd(a.tile_counter, 1u);
+		if (owner) {
+#pragma unroll
+			for (int i = 0; i < HALF; ++i) s_cnt[row_of(i) + pd] = 0;
+		}
+	}
+	K *__restrict__ kout = keys_out();
+	V *__restrict__ vout = vals_out();
 #pragma unroll
 	for (int i = 0; i < KPT; ++i) {
 		const int q = i * THREADS + tid;
@@ -934,6 +995,20 @@ radix_pass_tiles(const __grid_constant__ PassArgs<K, V> a, uint32_t num_tiles) {
 			if (HAS_V) vout[o] = sv[q];
 		}
 	}
+	if constexpr (MODE != kTilesLoop) return;
+	if (tid == 0) s_misc[0] = next;
+	// The staging area was written by plain stores; bulk copies write it next.
+	if constexpr (BULK) dev::fence_proxy_async();
+	__syncthreads();
+	t = s_misc[0];
+	if (t >= num_tiles) return;
+	parity ^= 1;
+	if (tid == 0 && (size_t)(t + 1) * TILE <= a.n) {
+		const K *ki = keys_in();
+		const V *vi = vals_in();
+		if (bulk_ok_for(ki, vi)) issue(ki, vi, t);
+	}
+	} while (MODE == kTilesLoop);
 }
 
 // ------------------------------------------------- small sorts in a cluster
@@ -1217,13 +1292,31 @@ cudaError_t launch_upsweep(int passes, cudaStream_t s, const K *keys, size_t n,
 	}
 }
 
-template <typename K, typename V, bool HAS_V, typename TC, bool GROUPED>
+// Passes of at least three waves of tiles run as resident CTAs that take tile
+// after tile: no gaps between CTAs, and a pass that the plan skips costs one
+// wave of empty CTAs instead of one per tile (2^28 equal keys 353 -> 178 us a
+// sort). Below, one CTA a tile is faster (u32 keys, us, one / loop: 5 x 10^6
+// 113 / 127, 10^7 192 / 192, 1.4 x 10^7 230 / 226; u64 4 x 10^6 228 / 239, 5 x 10^7
+// 1850 / 1771; (u64, u32) 5 x 10^6 390 / 401, 2^25 1843 / 1807).
+constexpr size_t kLoopWaves = 3;
+template <typename TC>
+bool loop_tiles(size_t n, CCLContext *ctx) {
+	return (n + TC::kTile - 1) / TC::kTile >= kLoopWaves * TC::kMinBlocks * ctx->sm_count;
+}
+template <typename TC, int MODE>
+unsigned pass_grid(size_t ctiles, CCLContext *ctx) {
+	return (unsigned)(MODE == kTilesLoop ? std::min<size_t>(ctiles,
+		(size_t)TC::kMinBlocks * ctx->sm_count) : ctiles);
+}
+
+template <typename K, typename V, bool HAS_V, typename TC, int MODE>
 cudaError_t sort_tiles(const K *src, K *dst, V *vals, size_t n, int passes,
 	CCLContext *ctx, cudaStream_t s, GError **err) {
-	// One CTA per tile of TC's size.
+	// Tiles of TC's size.
 	const size_t ctiles = (n + TC::kTile - 1) / TC::kTile;
+	const unsigned grid = pass_grid<TC, MODE>(ctiles, ctx);
 	const size_t smem = tiles_smem<K, V, HAS_V, TC::kThreads, TC::kKpt>();
-	auto kern = radix_pass_tiles<K, V, HAS_V, TC::kThreads, TC::kKpt, TC::kMinBlocks, GROUPED>;
+	auto kern = radix_pass_tiles<K, V, HAS_V, TC::kThreads, TC::kKpt, TC::kMinBlocks, MODE>;
 	cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
 		(int)smem);
 	if (e != cudaSuccess) {
@@ -1236,7 +1329,7 @@ cudaError_t sort_tiles(const K *src, K *dst, V *vals, size_t n, int passes,
 	const bool copy_back = in_place && passes == 1;
 	// Scratch: [control][status0][status1][alt keys][alt vals], a status row
 	// per tile (and per group of tiles).
-	const size_t status_words = (ctiles + (GROUPED ? (ctiles + kGroup - 1) / kGroup : 0)) * kRadix;
+	const size_t status_words = (ctiles + (MODE == kTilesGrouped ? (ctiles + kGroup - 1) / kGroup : 0)) * kRadix;
 	const size_t off_st0 = (control_words(passes) * 4 + 255) / 256 * 256;
 	const size_t off_st1 = off_st0 + status_words * 4;
 	const size_t off_keys = (off_st1 + status_words * 4 + 255) / 256 * 256;
@@ -1275,7 +1368,7 @@ cudaError_t sort_tiles(const K *src, K *dst, V *vals, size_t n, int passes,
 		pa.shift = p * kRadixBits;
 		KernelTimer t("satradix_onesweep", s,
 			2.0 * (double)n * (sizeof(K) + (HAS_V ? sizeof(V) : 0)));
-		e = launch_chained(kern, (unsigned)ctiles, TC::kThreads, smem, s, 1, pa, (uint32_t)ctiles);
+		e = launch_chained(kern, grid, TC::kThreads, smem, s, 1, pa, (uint32_t)ctiles);
 		t.stop();
 	}
 	if (copy_back && e == cudaSuccess) {
@@ -1403,11 +1496,13 @@ cudaError_t sort_typed(const void *src, void *dst, void *vals, size_t n, int sor
 	// tiles.
 	const size_t sms = (size_t)ctx->sm_count;
 	auto fits = [&](size_t tile) { return (n + tile - 1) / tile <= sms; };
-	auto go = [&](auto tc, auto grouped) {
-		return sort_tiles<K, V, HAS_V, decltype(tc), decltype(grouped)::value>(ks, kd, v, n, passes,
+	auto go = [&](auto tc, auto mode) {
+		return sort_tiles<K, V, HAS_V, decltype(tc), decltype(mode)::value>(ks, kd, v, n, passes,
 			ctx, s, err);
 	};
-	using Yes = std::true_type;
+	using Yes = std::integral_constant<int, kTilesGrouped>;
+	using One = std::integral_constant<int, kTilesOne>;
+	using Loop = std::integral_constant<int, kTilesLoop>;
 	using P1 = TilesCfgPart<K, V, HAS_V, 1>;
 	using P2 = TilesCfgPart<K, V, HAS_V, 2>;
 	using P4 = TilesCfgPart<K, V, HAS_V, 4>;
@@ -1418,7 +1513,7 @@ cudaError_t sort_typed(const void *src, void *dst, void *vals, size_t n, int sor
 	if (fits(P4::kTile)) return go(P4(), Yes());
 	if (fits(P6::kTile)) return go(P6(), Yes());
 	if (n <= Big::kTile * kGroupedTiles<Big::kWords>) return go(Big(), Yes());
-	return go(Big(), std::false_type());
+	return loop_tiles<Big>(n, ctx) ? go(Big(), Loop()) : go(Big(), One());
 }
 
 // Stable partition of n keys by the top 8 of their sort_bits low bits:
@@ -1431,9 +1526,10 @@ cudaError_t msd_partition_typed(const K *keys_in, K *keys_out, size_t n, int sor
 	using TC = TilesCfg<K, uint32_t, false>;
 	const int shift = sort_bits - kRadixBits;
 	const size_t ctiles = (n + TC::kTile - 1) / TC::kTile;
+	const unsigned grid = pass_grid<TC, kTilesLoop>(ctiles, ctx);
 	const size_t smem = tiles_smem<K, uint32_t, false, TC::kThreads, TC::kKpt>();
 	auto kern = radix_pass_tiles<K, uint32_t, false, TC::kThreads, TC::kKpt, TC::kMinBlocks,
-		false>;
+		kTilesLoop>;
 	cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
 		(int)smem);
 	if (e != cudaSuccess) {
@@ -1470,7 +1566,7 @@ cudaError_t msd_partition_typed(const K *keys_in, K *keys_out, size_t n, int sor
 		pa.n = n;
 		pa.shift = shift;
 		KernelTimer t("satradix_onesweep", s, 2.0 * (double)n * sizeof(K));
-		e = launch_chained(kern, (unsigned)ctiles, TC::kThreads, smem, s, 1, pa, (uint32_t)ctiles);
+		e = launch_chained(kern, grid, TC::kThreads, smem, s, 1, pa, (uint32_t)ctiles);
 		t.stop();
 	}
 	if (e == cudaSuccess)

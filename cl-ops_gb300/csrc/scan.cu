@@ -48,8 +48,8 @@ __device__ __forceinline__ Acc shfl_up(Acc v, int d) {
 }
 
 // Persistent CTAs (one per resident slot) take tiles in order from an
-// atomic counter. Per tile: the sums of the tile already in shared memory
-// and publication of its aggregate; then, while warp 0 looks back, every
+// atomic counter. Per tile: the sums of the tile already in registers and
+// publication of its aggregate; then, while warp 0 looks back, every
 // warp issues the loads of the CTA's next tile (claimed at the top of the
 // iteration) into registers and sums them, so the next tile's aggregate is
 // published as soon as the lookback ends -- before this tile's outputs are
