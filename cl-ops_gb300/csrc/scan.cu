@@ -7,15 +7,17 @@
 // Integer addition is associative, so the result is bit-identical to the
 // reference's work-group Blelloch trees whatever the summation order.
 //
-// Layout (scan_rows.cuh): tiles of 8192 elements, 256 threads, held in
-// registers as rows of whole vectors per lane; a row's scan is a warp scan of
+// Layout (scan_rows.cuh): tiles of 4096 to 16384 elements by type and size
+// (ScanBig and the ones after it), held in registers as rows of whole vectors per lane; a row's scan is a warp scan of
 // the lanes' run sums. Tiles take ids from an atomic counter (so a tile only
 // ever waits on tiles already running), publish their aggregate, then warp 0
 // looks back over a 64-tile window per round trip until it meets an
 // inclusive prefix. Status words carry their own ready bits, so neither side
 // needs a memory fence. Every wait is bounded. Staging the tile in shared
-// memory (a lane scanning 16 consecutive elements, seven shared wavefronts
-// per 32 elements for uint -> ulong) took 589 us at 2^28 against 519.
+// memory (scan_staged.cuh: a lane scans 16 consecutive elements, seven shared
+// wavefronts per 32 elements for uint -> ulong) takes 589 us at 2^28 against
+// 517; it stays for the types and alignments the rows are slow at
+// (staged_scan).
 //
 // HBM roofline: sizeof(in) + sizeof(out) bytes per element (12 B for
 // uint -> ulong), plus 32 B of tile status per tile.
@@ -28,6 +30,7 @@
 #include "dev_common.cuh"
 #include "launch.h"
 #include "scan_rows.cuh"
+#include "scan_staged.cuh"
 #include "scan_status.cuh"
 #include "timing.h"
 
@@ -60,8 +63,14 @@ __device__ __forceinline__ Acc shfl_up(Acc v, int d) {
 template <typename InT, typename OutT, int THREADS, int TILE, int MINB, bool KEEP = false>
 struct ScanCfg {
 	static constexpr int kThreads = THREADS, kTile = TILE, kMinBlocks = MINB;
-	static constexpr bool kKeepShared = KEEP;
+	static constexpr bool kKeepShared = KEEP, kStaged = false;
 	using R = Rows<InT, OutT, THREADS, TILE>;
+};
+// The staged kernel's shape.
+template <typename InT, typename OutT>
+struct ScanStaged {
+	static constexpr int kThreads = scantile::kThreads, kTile = scantile::kTile;
+	static constexpr bool kStaged = true;
 };
 // Sums of one or two bytes, or narrower than the input: one shape for all.
 template <typename InT, typename OutT>
@@ -102,6 +111,28 @@ using ScanSmall = If<kOneShape<InT, OutT>, ScanBig<InT, OutT>,
 // ulong: 8.8 us with a memset and a 256-thread tile, 3.9 so).
 template <typename InT, typename OutT>
 using ScanOne = If<kOneShape<InT, OutT>, ScanBig<InT, OutT>, ScanCfg<InT, OutT, 1024, 8192, 1>>;
+
+// Scans that take the staged kernel (scan_staged.cuh), which moves whole lines
+// whatever the types and the alignment. A row's lanes are kE elements apart:
+// with sums narrower than the input that is 64 to 256 bytes, and arrays that
+// are not 16-byte aligned are taken element by element at that distance. us,
+// rows / staged (the staged kernel before the rows came, unchained, in brackets):
+//   sums of 1 or 2 bytes or narrower than the input: uint -> uchar 2^20 8.3 / 8.2
+//   (12.9), 2^22 15.2 / 13.2, 2^28 627 / 322 (333); ushort -> ushort 2^22 10.9 /
+//   13.3, 2^23 18.7 / 17.9, 2^28 467 / 351 (361); ulong -> uint 2^22 16.8 / 16.0,
+//   6 x 10^6 21.4 / 22.5, 2^24 55 / 46, 2^28 787 / 614 (619);
+//   inputs of 1 or 2 bytes, sums of 8 (too few bytes in flight with two CTAs an
+//   SM): uchar 12 x 10^6 29.2 / 30.0, 2^24 36.5 / 36.2, 2^28 486 / 440 (447);
+//   unaligned: uint -> uint 2^18 6.5 / 7.5, 2^19 7.1 / 8.3, 2^20 11.9 / 10.7, 2^26
+//   360 / 204 (213); uchar -> ulong 2^26 666 / 201 (209); sums of the first kind
+//   at every size (ulong -> uint 20000 9.6 / 7.1).
+template <typename InT, typename OutT>
+bool staged_scan(size_t n, int vec) {
+	constexpr size_t kM = (size_t)1 << 20;
+	if (!(vec & 1)) return kOneShape<InT, OutT> || n > kM / 2;
+	if (kOneShape<InT, OutT>) return n > (sizeof(InT) == 4 ? kM : 8 * kM);
+	return sizeof(OutT) == 8 && sizeof(InT) <= 2 && n > 16 * kM;
+}
 
 template <typename InT, typename OutT, typename CFG>
 __global__ void __launch_bounds__(CFG::kThreads, CFG::kMinBlocks)
@@ -304,9 +335,15 @@ __global__ void __launch_bounds__(256) copy_words(char *dst, const char *src, si
 	for (size_t i = vecs * 16 + first; i < bytes; i += stride) dst[i] = src[i];
 }
 
-template <typename CFG>
+template <typename InT, typename OutT, typename CFG>
+constexpr auto scan_kernel() {
+	if constexpr (CFG::kStaged) return &scanstaged::scan_staged<InT, OutT>;
+	else return &scan_lookback<InT, OutT, CFG>;
+}
+template <typename InT, typename OutT, typename CFG>
 constexpr size_t scan_shared() {
-	return CFG::kKeepShared ? (size_t)CFG::kThreads * CFG::R::kRows * CFG::R::kWords * 4 : 0;
+	if constexpr (CFG::kStaged) return scantile::scan_smem<InT, OutT>();
+	else return CFG::kKeepShared ? (size_t)CFG::kThreads * CFG::R::kRows * CFG::R::kWords * 4 : 0;
 }
 
 // Per device and type pair, once: records the kernel's resident CTAs per SM.
@@ -325,12 +362,12 @@ cudaError_t scan_prepare(int *per_sm) {
 		std::lock_guard<std::mutex> lk(mu);
 		v = cached[dev].load(std::memory_order_relaxed);
 		if (v == 0) {
-			if (scan_shared<CFG>() > 48 * 1024)
-				e = cudaFuncSetAttribute(scan_lookback<InT, OutT, CFG>,
-					cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scan_shared<CFG>());
+			if (scan_shared<InT, OutT, CFG>() > 48 * 1024)
+				e = cudaFuncSetAttribute(scan_kernel<InT, OutT, CFG>(),
+					cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scan_shared<InT, OutT, CFG>());
 			if (e == cudaSuccess)
-				e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, scan_lookback<InT, OutT, CFG>,
-				CFG::kThreads, scan_shared<CFG>());
+				e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, scan_kernel<InT, OutT, CFG>(),
+					CFG::kThreads, scan_shared<InT, OutT, CFG>());
 			if (e != cudaSuccess) return e;
 			if (v < 1) v = 1;
 			cached[dev].store(v, std::memory_order_release);
@@ -364,13 +401,13 @@ cudaError_t launch_scan_cfg(const void *in, void *out, size_t n, CCLContext *ctx
 		set_error(err, CLO_ERROR_ARGS, "Scan of %zu elements is too large", n);
 		return cudaErrorInvalidValue;
 	}
-	// One tile needs no statuses.
+	// One tile of rows needs no statuses.
 	const size_t status_bytes = tiles * Slots<Acc>::kPerTile * sizeof(uint64_t);
 	const size_t bytes = status_bytes + 16;
 	char *tmp = nullptr;
 	TileStatus ts = {nullptr, nullptr};
 	cudaError_t e = cudaSuccess;
-	if (tiles > 1) {
+	if (tiles > 1 || CFG::kStaged) {
 		tmp = (char *)tmp_alloc(ctx, bytes, s, err);
 		if (!tmp) return cudaErrorMemoryAllocation;
 		ts.words = (uint64_t *)tmp;
@@ -381,9 +418,9 @@ cudaError_t launch_scan_cfg(const void *in, void *out, size_t n, CCLContext *ctx
 	if (e == cudaSuccess) e = scan_prepare<InT, OutT, CFG>(&per_sm);
 	if (e == cudaSuccess) {
 		KernelTimer t("scan_lookback", s, (double)n * (sizeof(InT) + sizeof(OutT)));
-		e = launch_chained(scan_lookback<InT, OutT, CFG>, scan_grid(tiles, per_sm, ctx->sm_count),
-			CFG::kThreads, scan_shared<CFG>(), s, 1, (const InT *)in, (OutT *)out, n, ts, ctx->d_status,
-			scan_vec(in, out), debug_skip_tile, carry_in, carry_out);
+		e = launch_chained(scan_kernel<InT, OutT, CFG>(), scan_grid(tiles, per_sm, ctx->sm_count),
+			CFG::kThreads, scan_shared<InT, OutT, CFG>(), s, 1, (const InT *)in, (OutT *)out, n, ts,
+			ctx->d_status, scan_vec(in, out), debug_skip_tile, carry_in, carry_out);
 		t.stop();
 		count_launches(1);
 	}
@@ -399,6 +436,7 @@ cudaError_t launch_scan(const void *in, void *out, size_t n, CCLContext *ctx,
 		return launch_scan_cfg<InT, OutT, decltype(cfg)>(in, out, n, ctx, s, err, debug_skip_tile, ci,
 			co);
 	};
+	if (staged_scan<InT, OutT>(n, scan_vec(in, out))) return go(ScanStaged<InT, OutT>());
 	if (n <= ScanOne<InT, OutT>::kTile) return go(ScanOne<InT, OutT>());
 	if (n <= kSmallMax) return go(ScanSmall<InT, OutT>());
 	if (n <= kMidMax) return go(ScanMid<InT, OutT>());
@@ -520,13 +558,18 @@ struct CurrentDevice {
 // Opts every (element, sum) instantiation of the scan kernel into its
 // shared memory and caches its occupancy, so that no later call does any
 // set-up work, whatever its type pair.
+template <typename InT, typename OutT>
+cudaError_t noalloc_prepare() {
+	int v = 0;
+	cudaError_t e = scan_prepare<InT, OutT, ScanBig<InT, OutT>>(&v);
+	return e == cudaSuccess ? scan_prepare<InT, OutT, ScanStaged<InT, OutT>>(&v) : e;
+}
 template <typename InT>
 cudaError_t noalloc_prepare_in() {
-	int v = 0;
-	cudaError_t e = scan_prepare<InT, uint8_t, ScanBig<InT, uint8_t>>(&v);
-	if (e == cudaSuccess) e = scan_prepare<InT, uint16_t, ScanBig<InT, uint16_t>>(&v);
-	if (e == cudaSuccess) e = scan_prepare<InT, uint32_t, ScanBig<InT, uint32_t>>(&v);
-	if (e == cudaSuccess) e = scan_prepare<InT, uint64_t, ScanBig<InT, uint64_t>>(&v);
+	cudaError_t e = noalloc_prepare<InT, uint8_t>();
+	if (e == cudaSuccess) e = noalloc_prepare<InT, uint16_t>();
+	if (e == cudaSuccess) e = noalloc_prepare<InT, uint32_t>();
+	if (e == cudaSuccess) e = noalloc_prepare<InT, uint64_t>();
 	return e;
 }
 
@@ -570,12 +613,11 @@ uint64_t *noalloc_scratch(int ordinal, GError **err) {
 	return g_noalloc_addr[ordinal];
 }
 
-template <typename InT, typename OutT>
-cudaError_t launch_scan_noalloc(const void *in, void *out, size_t n,
+template <typename InT, typename OutT, typename CFG>
+cudaError_t launch_scan_noalloc_cfg(const void *in, void *out, size_t n,
 	uint64_t *scratch, int *dev_status, int sm_count, cudaStream_t s) {
 	using Acc = typename std::conditional<(sizeof(OutT) <= 4), uint32_t,
 		uint64_t>::type;
-	using CFG = ScanBig<InT, OutT>;
 	const size_t tiles = (n + CFG::kTile - 1) / CFG::kTile;
 	TileStatus ts;
 	ts.words = scratch;
@@ -589,11 +631,21 @@ cudaError_t launch_scan_noalloc(const void *in, void *out, size_t n,
 	int per_sm = 1;
 	e = scan_prepare<InT, OutT, CFG>(&per_sm);
 	if (e != cudaSuccess) return e;
-	scan_lookback<InT, OutT, CFG><<<scan_grid(tiles, per_sm, sm_count), CFG::kThreads, scan_shared<CFG>(),
-		s>>>((const InT *)in, (OutT *)out, n, ts, dev_status, scan_vec(in, out), -1, nullptr,
-		nullptr);
+	scan_kernel<InT, OutT, CFG>()<<<scan_grid(tiles, per_sm, sm_count), CFG::kThreads,
+		scan_shared<InT, OutT, CFG>(), s>>>((const InT *)in, (OutT *)out, n, ts, dev_status,
+		scan_vec(in, out), -1, nullptr, nullptr);
 	count_launches(1);
 	return cudaGetLastError();
+}
+
+template <typename InT, typename OutT>
+cudaError_t launch_scan_noalloc(const void *in, void *out, size_t n,
+	uint64_t *scratch, int *dev_status, int sm_count, cudaStream_t s) {
+	return staged_scan<InT, OutT>(n, scan_vec(in, out))
+		? launch_scan_noalloc_cfg<InT, OutT, ScanStaged<InT, OutT>>(in, out, n, scratch, dev_status,
+			sm_count, s)
+		: launch_scan_noalloc_cfg<InT, OutT, ScanBig<InT, OutT>>(in, out, n, scratch, dev_status,
+			sm_count, s);
 }
 
 template <typename InT>

@@ -1,9 +1,10 @@
 // Register layout of the plain scan's tiles: a warp owns a stretch of
 // consecutive elements in rows of 32 x kE: in row r lane l
 // holds elements kE l .. kE l + kE - 1, kE being as many as fill a 32-byte
-// store of outputs. Loads and stores are whole coalesced vectors between
-// global memory and registers, and a row's scan is a warp scan of the lanes'
-// sums: nothing is staged in shared memory.
+// store of outputs. Loads and stores are whole vectors between global memory
+// and registers, and a row's scan is a warp scan of the lanes' sums: nothing
+// is transposed through shared memory (some shapes park a tile's registers
+// there, scan.cu).
 #pragma once
 
 #include <stddef.h>
@@ -32,7 +33,7 @@ struct Rows {
 		else return (InT)(uint8_t)(w[r][e / 4] >> (8 * (e % 4)));
 	}
 
-	// The warp's 1024 elements at p, all valid, as vectors: 32 bytes where
+	// The warp's kWarpElems elements at p, all valid, as vectors: 32 bytes where
 	// `wide` (p 32-byte aligned), else 16 (p 16-byte aligned).
 	__device__ __forceinline__ void load(const InT *p, int lane, bool wide) {
 #pragma unroll

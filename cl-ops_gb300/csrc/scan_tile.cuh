@@ -1,4 +1,4 @@
-// Tile layout of the segmented scan:
+// Tile layout of the segmented scan and of the staged plain scan:
 // 8192-element tiles, 256 threads; each warp owns 1024 consecutive
 // elements as two blocks of 512, lane l holding elements 16 l .. 16 l + 15
 // of each block. A block moves between global and shared memory with

@@ -1,0 +1,48 @@
+"""Which kernels the library's calls launch, over a CUDA runtime that launches
+nothing."""
+import pytest
+
+import fake_cuda
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    return fake_cuda.load(tmp_path_factory.mktemp("fake"))
+
+
+def _names(fake, call):
+    fake.lib.fake_reset(0)
+    call()
+    return [x[0] for x in fake_cuda.launches(fake)]
+
+
+# Sums of one or two bytes or narrower than the input, 8-byte sums of one or
+# two bytes and unaligned arrays leave the register rows where those are slow
+# (some of them took twice the time there).
+U8, U16, U32, U64 = 1, 3, 5, 7
+M = 1 << 20
+
+
+@pytest.mark.parametrize("i,o,offset,n,staged", [
+    (U32, U64, 0, 1 << 28, False), (U32, U32, 0, 1 << 28, False), (U64, U64, 0, 1 << 28, False),
+    (U8, U32, 0, 1 << 28, False), (U16, U32, 0, 1 << 28, False),
+    (U8, U8, 0, 8 * M, False), (U8, U8, 0, 8 * M + 1, True), (U16, U16, 0, 1 << 28, True),
+    (U32, U8, 0, M, False), (U32, U16, 0, M + 1, True), (U64, U32, 0, 1 << 26, True),
+    (U8, U64, 0, 16 * M, False), (U8, U64, 0, 16 * M + 1, True), (U16, U64, 0, 1 << 28, True),
+    (U32, U64, 8, M // 2, False), (U32, U64, 8, M // 2 + 1, True), (U8, U32, 4, 1 << 26, True),
+    (U64, U32, 8, 5000, True), (U64, U64, 16, 1 << 26, False),
+])
+def test_scan_route(fake, i, o, offset, n, staged):
+    ctx = fake.Context(0)
+    q = fake.Queue(ctx)
+    sc = fake.Scanner(ctx, i, o)
+    wrap = lambda at: fake.call(fake.lib.ccl_buffer_new_wrap, ctx.h, at, 8 * n)
+    a, b = wrap(1 << 40), wrap((1 << 41) + offset)
+    names = _names(fake, lambda: fake.call(fake.lib.clo_scan_with_device_data, sc.h, q.h, None, a,
+                                           b, n, 0))
+    scans = [x for x in names if "clear" not in x]
+    assert len(scans) == 1 and ("scan_staged" in scans[0]) == staged, names
+    for x in (a, b):
+        fake.lib.ccl_buffer_destroy(x)
+    for x in (sc, q, ctx):
+        x.destroy()
