@@ -343,19 +343,43 @@ radix_count16(const uint16_t *__restrict__ keys, size_t n, size_t per_cta,
 		const uint4 *v4 = reinterpret_cast<const uint4 *>(keys + v0);
 		constexpr int U = (kC16Step / 8 + kC16Threads - 1) / kC16Threads;  // 4
 		uint4 v[U];
+		auto held = [&](int u) { return threadIdx.x + u * kC16Threads < nv; };
 #pragma unroll
 		for (int u = 0; u < U; ++u)
-			if (threadIdx.x + u * kC16Threads < nv) v[u] = dev::ld_stream_v4(v4 + threadIdx.x + u * kC16Threads);
+			if (held(u)) v[u] = dev::ld_stream_v4(v4 + threadIdx.x + u * kC16Threads);
+		auto one_key = [](const uint4 &x) {
+			return x.x == x.y && x.x == x.z && x.x == x.w && x.x >> 16 == (x.x & 0xFFFFu);
+		};
+		auto count_all = [&](const uint4 &x) {
+			const uint32_t w[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-		for (int u = 0; u < U; ++u)
-			if (threadIdx.x + u * kC16Threads < nv) {
-				const uint32_t w[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+			for (int q = 0; q < 4; ++q) {
+				count(w[q] & 0xFFFFu);
+				count(w[q] >> 16);
+			}
+		};
+		// Where a thread's first eight keys are one key (sorted keys, few
+		// values) its warp looks for such vectors and adds them up before
+		// the shared counter, on which the lanes' adds would queue: us, 2^26
+		// equal keys 293 without, sorted ones 296.
+		if (__any_sync(0xffffffffu, held(0) && one_key(v[0]))) {
 #pragma unroll
-				for (int q = 0; q < 4; ++q) {
-					count(w[q] & 0xFFFFu);
-					count(w[q] >> 16);
+			for (int u = 0; u < U; ++u) {
+				const bool same = held(u) && one_key(v[u]);
+				const uint32_t m = __ballot_sync(0xffffffffu, same);
+				if (same) {
+					const uint32_t k = v[u].x & 0xFFFFu, peers = __match_any_sync(m, k);
+					if ((peers & dev::lanemask_lt()) == 0)
+						atomicAdd(c16 + (k >> 1), 8u * __popc(peers) << ((k & 1u) << 4));
+				} else if (held(u)) {
+					count_all(v[u]);
 				}
 			}
+		} else {
+#pragma unroll
+			for (int u = 0; u < U; ++u)
+				if (held(u)) count_all(v[u]);
+		}
 		for (size_t i = v0 + (size_t)nv * 8 + threadIdx.x; i < e; i += kC16Threads) count(keys[i]);
 		__syncthreads();
 		if (e < finish) {
