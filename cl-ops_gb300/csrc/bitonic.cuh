@@ -588,11 +588,11 @@ __device__ __forceinline__ void smem_stage_tail(T *s, uint32_t tile_n, int j,
 	}
 }
 
-// first: stages 1..t of every tile of 2^t elements; otherwise steps t..1 of
+// FIRST: stages 1..t of every tile of 2^t elements; otherwise steps t..1 of
 // `stage` (> t).
-template <typename T>
+template <typename T, bool FIRST>
 __global__ void __launch_bounds__(kRoundThreads, sizeof(T) <= 4 ? 3 : 2)
-bitonic_rounds(T *data, int t, int stage, int maxg, bool first) {
+bitonic_rounds(T *data, int t, int stage, int maxg) {
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	T *s = reinterpret_cast<T *>(smem_raw);
 	const uint32_t tile_n = 1u << t;
@@ -600,13 +600,19 @@ bitonic_rounds(T *data, int t, int stage, int maxg, bool first) {
 	T *g = data + tile_base;
 	for (uint32_t i = threadIdx.x; i < tile_n; i += blockDim.x) s[spad(i)] = g[i];
 	__syncthreads();
-	if (first) {
-		for (int st = 1; st < t; ++st)
-			smem_stage_tail(s, tile_n, st, maxg, [st](uint32_t i) { return (bool)((i >> st) & 1); });
-		stage = t;
+	if constexpr (FIRST) {
+		for (int st = 1; st <= t; ++st) {
+			if (st < t) {
+				smem_stage_tail(s, tile_n, st, maxg, [st](uint32_t i) { return (bool)((i >> st) & 1); });
+			} else {
+				const bool d = (tile_base >> st) & 1;
+				smem_stage_tail(s, tile_n, st, maxg, [d](uint32_t) { return d; });
+			}
+		}
+	} else {
+		const bool d = (tile_base >> stage) & 1;
+		smem_stage_tail(s, tile_n, t, maxg, [d](uint32_t) { return d; });
 	}
-	const bool d = (tile_base >> stage) & 1;
-	smem_stage_tail(s, tile_n, t, maxg, [d](uint32_t) { return d; });
 	for (uint32_t i = threadIdx.x; i < tile_n; i += blockDim.x) g[i] = s[spad(i)];
 }
 
@@ -730,8 +736,11 @@ cudaError_t run_rounds(T *d, int logN, int max_ps, int max_sfs, cudaStream_t s,
 	const uint32_t tile_n = 1u << t;
 	const size_t smem = (size_t)(tile_n + tile_n / 32 + 1) * sizeof(T);
 	const unsigned threads = std::min<uint32_t>(kRoundThreads, std::max<uint32_t>(tile_n / 2, 32));
-	cudaError_t e = cudaFuncSetAttribute(bitonic_rounds<T>,
+	cudaError_t e = cudaFuncSetAttribute(bitonic_rounds<T, true>,
 		cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+	if (e == cudaSuccess)
+		e = cudaFuncSetAttribute(bitonic_rounds<T, false>,
+			cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 	const size_t tiles = N >> t;
 	const double pass_bytes = 2.0 * (double)N * sizeof(T);
 	for (int stage = t; stage <= logN && e == cudaSuccess; ++stage) {
@@ -739,7 +748,8 @@ cudaError_t run_rounds(T *d, int logN, int max_ps, int max_sfs, cudaStream_t s,
 		if (!first) e = global_passes<T>(d, N, stage, t, gmaxg, pass_bytes, s, launches);
 		if (e != cudaSuccess) break;
 		KernelTimer tm(first ? "abitonic_tile_sort" : "abitonic_tile_finish", s, pass_bytes);
-		bitonic_rounds<T><<<(unsigned)tiles, threads, smem, s>>>(d, t, stage, maxg, first);
+		auto kern = first ? bitonic_rounds<T, true> : bitonic_rounds<T, false>;
+		kern<<<(unsigned)tiles, threads, smem, s>>>(d, t, stage, maxg);
 		tm.stop();
 		launches++;
 		e = cudaGetLastError();
