@@ -7,7 +7,7 @@
 namespace clo {
 
 cudaError_t bitonic_sort(const void *src, void *dst, size_t n, CloType type, int max_ps,
-	int max_sfs, CCLContext *ctx, cudaStream_t s, GError **err) {
+	int max_sfs, BitonicUser user, CCLContext *ctx, cudaStream_t s, GError **err) {
 	const size_t eb = clo_type_sizeof(type);
 	if (eb != 1 && eb != 2 && eb != 4 && eb != 8) {
 		set_error(err, CLO_ERROR_ARGS, "Unsupported element type %d", (int)type);
@@ -27,10 +27,10 @@ cudaError_t bitonic_sort(const void *src, void *dst, size_t n, CloType type, int
 	}
 	if (n < 2) return cudaSuccess;
 	switch (eb) {
-	case 1: return bitonic::sort_width1(src, dst, n, type, max_ps, max_sfs, ctx, s, err);
-	case 2: return bitonic::sort_width2(src, dst, n, type, max_ps, max_sfs, ctx, s, err);
-	case 4: return bitonic::sort_width4(src, dst, n, type, max_ps, max_sfs, ctx, s, err);
-	default: return bitonic::sort_width8(src, dst, n, type, max_ps, max_sfs, ctx, s, err);
+	case 1: return bitonic::sort_width1(src, dst, n, type, max_ps, max_sfs, user, ctx, s, err);
+	case 2: return bitonic::sort_width2(src, dst, n, type, max_ps, max_sfs, user, ctx, s, err);
+	case 4: return bitonic::sort_width4(src, dst, n, type, max_ps, max_sfs, user, ctx, s, err);
+	default: return bitonic::sort_width8(src, dst, n, type, max_ps, max_sfs, user, ctx, s, err);
 	}
 }
 

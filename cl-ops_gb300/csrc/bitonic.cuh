@@ -623,6 +623,15 @@ __global__ void fill_value(T *p, size_t n, T v) {
 }
 
 // ------------------------------------------------------------- launches
+// What the per-kernel timing calls them, by BitonicUser.
+struct TimerNames {
+	const char *tile_sort, *global_steps, *tile_finish;
+};
+constexpr TimerNames kTimerNames[] = {
+	{"abitonic_tile_sort", "abitonic_global_steps", "abitonic_tile_finish"},
+	{"sbitonic_tile_sort", "sbitonic_global_steps", "sbitonic_tile_finish"},
+	{"satradix_tile_sort", "satradix_global_steps", "satradix_tile_finish"}};
+
 inline int ilog2(size_t v) {
 	int r = 0;
 	while (((size_t)1 << r) < v) ++r;
@@ -634,14 +643,14 @@ inline int ilog2(size_t v) {
 // not 5 + 1): a pass of few steps per thread is the slowest per byte.
 template <typename T>
 cudaError_t global_passes(T *d, size_t elems, int stage, int t, int maxg, double bytes,
-	cudaStream_t s, unsigned &launches) {
+	const TimerNames &names, cudaStream_t s, unsigned &launches) {
 	cudaError_t e = cudaSuccess;
 	for (int j = stage; j > t && e == cudaSuccess;) {
 		const int rem = j - t;
 		const int npass = (rem + maxg - 1) / maxg;
 		const int g = (rem + npass - 1) / npass;
 		const size_t groups = elems >> g;
-		KernelTimer tm("abitonic_global_steps", s, bytes);
+		KernelTimer tm(names.global_steps, s, bytes);
 		auto go = [&](auto G) {
 			constexpr int g_ = decltype(G)::value;
 			constexpr int V = 16 / sizeof(T);
@@ -683,8 +692,8 @@ constexpr int kGlobalSteps = sizeof(T) == 4 ? 7 : sizeof(T) == 1 ? 5 : 6;
 // The sort with one tile configuration. `work` holds N elements (it may be
 // `dst` when n == N; null when one tile holds everything).
 template <typename T, typename C>
-cudaError_t run_tiles(const T *src, T *dst, T *work, size_t n, int logN, cudaStream_t s,
-	unsigned &launches) {
+cudaError_t run_tiles(const T *src, T *dst, T *work, size_t n, int logN,
+	const TimerNames &names, cudaStream_t s, unsigned &launches) {
 	constexpr int K = C::kK;
 	const size_t N = (size_t)1 << logN;
 	const int TL = C::TL;
@@ -702,7 +711,7 @@ cudaError_t run_tiles(const T *src, T *dst, T *work, size_t n, int logN, cudaStr
 	const size_t parts = one ? (size_t)C::kCluster : N >> K;
 	const double pass_bytes = 2.0 * (double)N * sizeof(T);
 	{
-		KernelTimer tm("abitonic_tile_sort", s, pass_bytes);
+		KernelTimer tm(names.tile_sort, s, pass_bytes);
 		e = launch_chained(sort_k, (unsigned)parts, C::kThreads, C::kSmem, s, C::kCluster, src,
 			one ? dst : work, n, one ? n : N, std::min(logN, TL));
 		tm.stop();
@@ -711,10 +720,10 @@ cudaError_t run_tiles(const T *src, T *dst, T *work, size_t n, int logN, cudaStr
 	for (int stage = TL + 1; stage <= logN && e == cudaSuccess; ++stage) {
 		// A stage leaves blocks of padding alone as they are.
 		const size_t elems = ((n + ((size_t)1 << stage) - 1) >> stage) << stage;
-		e = global_passes<T>(work, elems, stage, TL, kGlobalSteps<T>, pass_bytes, s, launches);
+		e = global_passes<T>(work, elems, stage, TL, kGlobalSteps<T>, pass_bytes, names, s, launches);
 		if (e != cudaSuccess) break;
 		const bool last = stage == logN;
-		KernelTimer tf("abitonic_tile_finish", s, pass_bytes);
+		KernelTimer tf(names.tile_finish, s, pass_bytes);
 		e = launch_chained(fin_k, (unsigned)(elems >> K), C::kThreads, C::kSmem, s, C::kCluster,
 			(const T *)work, last ? dst : work, N, last ? n : N, stage);
 		tf.stop();
@@ -726,8 +735,8 @@ cudaError_t run_tiles(const T *src, T *dst, T *work, size_t n, int logN, cudaStr
 // Settings that bound the grouping: at most max_ps steps per round and tiles
 // of 2^max_sfs elements, on N elements in place.
 template <typename T>
-cudaError_t run_rounds(T *d, int logN, int max_ps, int max_sfs, cudaStream_t s,
-	unsigned &launches) {
+cudaError_t run_rounds(T *d, int logN, int max_ps, int max_sfs,
+	const TimerNames &names, cudaStream_t s, unsigned &launches) {
 	const size_t N = (size_t)1 << logN;
 	int t = std::min(sizeof(T) >= 8 ? 13 : 14, logN);
 	if (max_sfs >= 1 && max_sfs < t) t = max_sfs;
@@ -745,9 +754,9 @@ cudaError_t run_rounds(T *d, int logN, int max_ps, int max_sfs, cudaStream_t s,
 	const double pass_bytes = 2.0 * (double)N * sizeof(T);
 	for (int stage = t; stage <= logN && e == cudaSuccess; ++stage) {
 		const bool first = stage == t;
-		if (!first) e = global_passes<T>(d, N, stage, t, gmaxg, pass_bytes, s, launches);
+		if (!first) e = global_passes<T>(d, N, stage, t, gmaxg, pass_bytes, names, s, launches);
 		if (e != cudaSuccess) break;
-		KernelTimer tm(first ? "abitonic_tile_sort" : "abitonic_tile_finish", s, pass_bytes);
+		KernelTimer tm(first ? names.tile_sort : names.tile_finish, s, pass_bytes);
 		auto kern = first ? bitonic_rounds<T, true> : bitonic_rounds<T, false>;
 		kern<<<(unsigned)tiles, threads, smem, s>>>(d, t, stage, maxg);
 		tm.stop();
@@ -780,10 +789,11 @@ constexpr int kBigDoubleMin = 23;  // log2: 8-byte tiles of 2^13 from here
 
 template <typename T>
 cudaError_t sort_typed(const T *src, T *dst, size_t n, int max_ps, int max_sfs,
-	CCLContext *ctx, cudaStream_t s, GError **err) {
+	BitonicUser user, CCLContext *ctx, cudaStream_t s, GError **err) {
 	cudaError_t e = cudaSuccess;
 	const int logN = ilog2(n);
 	const size_t N = (size_t)1 << logN;
+	const TimerNames &names = kTimerNames[user];
 	unsigned launches = 0;
 	T *tmp = nullptr;
 	const int t0 = std::min(sizeof(T) >= 8 ? 13 : 14, logN);
@@ -803,19 +813,19 @@ cudaError_t sort_typed(const T *src, T *dst, size_t n, int max_ps, int max_sfs,
 			launches++;
 			e = cudaGetLastError();
 		}
-		if (e == cudaSuccess) e = run_rounds<T>(work, logN, max_ps, max_sfs, s, launches);
+		if (e == cudaSuccess) e = run_rounds<T>(work, logN, max_ps, max_sfs, names, s, launches);
 		if (e == cudaSuccess && tmp)
 			e = cudaMemcpyAsync(dst, tmp, n * sizeof(T), cudaMemcpyDeviceToDevice, s);
 	} else if (logN > SmallTile<T>::kK && logN <= kOneTile<T>) {
 		if constexpr (sizeof(T) <= 4)
-			e = run_tiles<T, ClusterTile<T>>(src, dst, work, n, logN, s, launches);
+			e = run_tiles<T, ClusterTile<T>>(src, dst, work, n, logN, names, s, launches);
 	} else {
 		bool big = false;
 		if constexpr (sizeof(T) == 8) {
 			big = logN >= kBigDoubleMin;
-			if (big) e = run_tiles<T, TileCfg<T, 13, 0, 4>>(src, dst, work, n, logN, s, launches);
+			if (big) e = run_tiles<T, TileCfg<T, 13, 0, 4>>(src, dst, work, n, logN, names, s, launches);
 		}
-		if (!big) e = run_tiles<T, SmallTile<T>>(src, dst, work, n, logN, s, launches);
+		if (!big) e = run_tiles<T, SmallTile<T>>(src, dst, work, n, logN, names, s, launches);
 	}
 	if (tmp) tmp_free(tmp, s);
 	count_launches(launches);

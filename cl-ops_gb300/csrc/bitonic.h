@@ -19,7 +19,7 @@ struct Half16 {
 // of one width.
 #define CLO_BITONIC_WIDTH(W) \
 	cudaError_t sort_width##W(const void *src, void *dst, size_t n, CloType type, int max_ps, \
-		int max_sfs, CCLContext *ctx, cudaStream_t s, GError **err);
+		int max_sfs, BitonicUser user, CCLContext *ctx, cudaStream_t s, GError **err);
 CLO_BITONIC_WIDTH(1)
 CLO_BITONIC_WIDTH(2)
 CLO_BITONIC_WIDTH(4)

@@ -5,10 +5,10 @@ namespace clo {
 namespace bitonic {
 
 cudaError_t sort_width8(const void *src, void *dst, size_t n, CloType type, int max_ps,
-	int max_sfs, CCLContext *ctx, cudaStream_t s, GError **err) {
+	int max_sfs, BitonicUser user, CCLContext *ctx, cudaStream_t s, GError **err) {
 	auto go = [&](auto t) {
 		using T = decltype(t);
-		return sort_typed<T>((const T *)src, (T *)dst, n, max_ps, max_sfs, ctx, s, err);
+		return sort_typed<T>((const T *)src, (T *)dst, n, max_ps, max_sfs, user, ctx, s, err);
 	};
 	switch (type) {
 	case CLO_LONG: return go(int64_t());

@@ -162,9 +162,11 @@ cudaError_t scan_exclusive_carry(const void *in, void *out, size_t n,
 // Non-power-of-two n is padded (in a temporary) with the type's maximum.
 // src's elements into dst, which may be src. max_ps bounds the steps grouped
 // per pass (4: no bound), max_sfs the largest step finished in shared memory
-// (0: no bound); neither changes the result.
+// (0: no bound); neither changes the result. The per-kernel timing names the
+// kernels by their sorter.
+enum BitonicUser { BITONIC_ABITONIC, BITONIC_SBITONIC, BITONIC_SATRADIX };
 cudaError_t bitonic_sort(const void *src, void *dst, size_t n, CloType type, int max_ps,
-	int max_sfs, CCLContext *ctx, cudaStream_t s, GError **err);
+	int max_sfs, BitonicUser user, CCLContext *ctx, cudaStream_t s, GError **err);
 
 // Rank-by-counting sort (stable, out of place): out[rank(i)] = in[i].
 // Optional values (val_bytes 0/4/8) follow their keys.

@@ -44,7 +44,8 @@ cudaError_t radix_sort(const void *src, void *dst, void *vals, size_t n, int key
 	// 101 / 80; keys of one and two bytes are faster by radix).
 	if (val_bytes == 0 && key_bytes >= 4 && sort_bits == 8 * key_bytes &&
 		n <= ((size_t)1 << (key_bytes == 8 ? 18 : 17)))
-		return bitonic_sort(src, dst, n, key_bytes == 8 ? CLO_ULONG : CLO_UINT, 4, 0, ctx, s, err);
+		return bitonic_sort(src, dst, n, key_bytes == 8 ? CLO_ULONG : CLO_UINT, 4, 0,
+			BITONIC_SATRADIX, ctx, s, err);
 	switch (key_bytes) {
 	case 1: return radix::sort<uint8_t>(src, dst, vals, n, val_bytes, sort_bits, ctx, s, err);
 	case 2: return radix::sort<uint16_t>(src, dst, vals, n, val_bytes, sort_bits, ctx, s, err);

@@ -425,8 +425,8 @@ CCLEvent *bitonic_sort_common(CloSort *s, CCLQueue *q, CCLBuffer *in,
 	// form, took 0.56 ms for 2^16 keys).
 	AbitonicData *d = (AbitonicData *)s->data;
 	cudaError_t e = clo::bitonic_sort(in->ptr, out->ptr, numel, s->elem_type,
-		d ? (int)d->max_ps : 4, d && d->max_sfs < 64 ? (int)d->max_sfs : 0, s->ctx, q->stream,
-		err);
+		d ? (int)d->max_ps : 4, d && d->max_sfs < 64 ? (int)d->max_sfs : 0,
+		simple ? clo::BITONIC_SBITONIC : clo::BITONIC_ABITONIC, s->ctx, q->stream, err);
 	if (e != cudaSuccess) return nullptr;
 	clo::event_end(ev);
 	return ev;

@@ -46,3 +46,32 @@ def test_scan_route(fake, i, o, offset, n, staged):
         fake.lib.ccl_buffer_destroy(x)
     for x in (sc, q, ctx):
         x.destroy()
+
+
+# The per-kernel timing names kernels by the sorter that was called, whichever
+# kernels it takes.
+@pytest.mark.parametrize("algo,code,n,names", [
+    ("satradix", U32, 1000, {"satradix_tile_sort": 1}),
+    ("satradix", U64, 1 << 16, {"satradix_tile_sort": 1, "satradix_global_steps": 5,
+                                "satradix_tile_finish": 5}),
+    ("satradix", U32, 1 << 20, {"satradix_upsweep": 1, "satradix_onesweep": 4}),
+    ("sbitonic", U32, 1000, {"sbitonic_tile_sort": 1}),
+    ("sbitonic", U32, 1 << 13, {"sbitonic_tile_sort": 1}),
+    ("abitonic", U32, 1 << 16, {"abitonic_tile_sort": 1, "abitonic_global_steps": 4,
+                                "abitonic_tile_finish": 4}),
+])
+def test_timing_names(fake, algo, code, n, names):
+    ctx = fake.Context(0)
+    q = fake.Queue(ctx)
+    s = fake.Sorter(ctx, algo, code)
+    a, b = fake.Buffer(ctx, 8 * n), fake.Buffer(ctx, 8 * n)
+    fake.lib.clo_gb300_timing_enable(1)
+    fake.lib.clo_gb300_timing_reset()
+    s.sort_device(q, a, n, buf_out=b)
+    got = {f"{x}_{k}": fake.kernel_timing(f"{x}_{k}")[2]
+           for x in ("satradix", "sbitonic", "abitonic")
+           for k in ("tile_sort", "global_steps", "tile_finish", "upsweep", "onesweep")}
+    fake.lib.clo_gb300_timing_enable(0)
+    assert {k: v for k, v in got.items() if v} == names
+    for x in (s, a, b, q, ctx):
+        x.destroy()
