@@ -122,8 +122,10 @@ bool type_is_signed(CloType t);
 // Stable LSD radix sort (onesweep) of n keys of key_bytes in {1,2,4,8} from
 // src into dst (which may be src), ascending by bits [0, sort_bits) of the
 // unsigned key pattern, carrying optional values of val_bytes in {0,4,8},
-// which are sorted in place. Passes whose digit is constant are skipped on
-// the device; nothing is read back.
+// which are sorted in place: with values src must be dst. A sort in place
+// takes an even number of 8-bit passes, or one. (Others are refused: their
+// last pass would write the buffer it reads.) Passes whose digit is constant
+// are skipped on the device; nothing is read back.
 cudaError_t radix_sort(const void *src, void *dst, void *vals, size_t n, int key_bytes,
 	int val_bytes, int sort_bits, CCLContext *ctx, cudaStream_t s, GError **err);
 

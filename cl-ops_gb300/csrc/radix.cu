@@ -22,6 +22,10 @@ cudaError_t radix_msd_partition(const void *keys_in, void *keys_out, size_t n, i
 
 cudaError_t radix_sort(const void *src, void *dst, void *vals, size_t n, int key_bytes,
 	int val_bytes, int sort_bits, CCLContext *ctx, cudaStream_t s, GError **err) {
+	if (val_bytes && src != dst) {
+		set_error(err, CLO_ERROR_ARGS, "satradix: values are sorted in place, with their keys");
+		return cudaErrorInvalidValue;
+	}
 	// Nothing to sort, or buffers that overlap in part: copied first.
 	const char *a = (const char *)src, *b = (const char *)dst;
 	const size_t bytes = n * (size_t)key_bytes;
@@ -36,6 +40,11 @@ cudaError_t radix_sort(const void *src, void *dst, void *vals, size_t n, int key
 		src = dst;
 	}
 	if (none) return cudaSuccess;
+	const int passes = sort_bits / radix::kRadixBits;
+	if (src == dst && passes > 1 && passes % 2) {
+		set_error(err, CLO_ERROR_ARGS, "satradix: %d passes in place", passes);
+		return cudaErrorInvalidValue;
+	}
 	// Small whole-key sorts without values: equal keys are the same bits, so
 	// any sort gives the stable one's result, and the bitonic tiles are faster
 	// while launches and latencies, not bytes, are what a sort costs (us,

@@ -1,5 +1,7 @@
 """Which kernels the library's calls launch, over a CUDA runtime that launches
 nothing."""
+import ctypes as C
+
 import pytest
 
 import fake_cuda
@@ -75,3 +77,31 @@ def test_timing_names(fake, algo, code, n, names):
     assert {k: v for k, v in got.items() if v} == names
     for x in (s, a, b, q, ctx):
         x.destroy()
+
+
+# The radix sort's launcher refuses what its passes would corrupt: values with
+# the keys going to another buffer, odd numbers of passes in place.
+@pytest.mark.parametrize("n", [5000, 100000, 1 << 24])
+@pytest.mark.parametrize("src,dst,vb,bits,ok", [
+    (0, 0, 4, 32, True), (0, 1, 0, 32, True), (0, 1, 0, 24, True), (0, 0, 0, 8, True),
+    (0, 0, 8, 64, True), (0, 1, 4, 32, False), (0, 1, 8, 16, False), (0, 0, 0, 24, False),
+    (0, 0, 4, 40, False), (0, 0.5, 0, 24, False)])
+def test_radix_sort_refusals(fake, n, src, dst, vb, bits, ok):
+    ctx = fake.Context(0)
+    q = fake.Queue(ctx)
+    f = fake.lib["_ZN3clo10radix_sortEPKvPvS2_miiiP11ccl_contextP11CUstream_stPP7_GError"]
+    f.restype = C.c_int
+    f.argtypes = [C.c_void_p] * 3 + [C.c_size_t] + [C.c_int] * 3 + [C.c_void_p] * 3
+    at = lambda x: int(1 << 40) + int(x * 8 * n) // 8 * 8
+    e = fake.err_ptr()
+    fake.lib.fake_reset(0)
+    # (The host memory that stands for the buffers is never touched.)
+    r = f(at(src), at(dst), (1 << 41) if vb else None, n, 8, vb, bits, ctx.h, None, C.addressof(e))
+    assert (r == 0) == ok and bool(e) != ok
+    if ok:
+        assert fake.lib.fake_launches() > 0
+    else:
+        assert fake.lib.fake_launches() == 0 and e.contents.code == fake.CLO_ERROR_ARGS
+        fake.lib.clo_error_free(e)
+    q.destroy()
+    ctx.destroy()
