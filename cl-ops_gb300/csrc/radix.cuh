@@ -202,7 +202,7 @@ __host__ __device__ constexpr int upw_pos_base(int p) {
 
 template <typename K, int PASSES>
 __global__ void __launch_bounds__(kUpwThreads, 1)
-radix_upsweep_w(const K *__restrict__ keys, size_t n, int base_shift, UpTail tail) {
+radix_upsweep_w(const K *keys, size_t n, int base_shift, UpTail tail) {
 	extern __shared__ __align__(16) uint32_t up_smem[];
 	for (int i = threadIdx.x; i < upw_pos_base(PASSES); i += kUpwThreads) up_smem[i] = 0;
 	dev::pdl_wait();
@@ -325,8 +325,8 @@ constexpr int kC16Threads = 1024, kC16Bins = 65536, kC16Step = 32760;
 constexpr size_t kC16Smem = kC16Bins * 2;
 
 __global__ void __launch_bounds__(kC16Threads, 1)
-radix_count16(const uint16_t *__restrict__ keys, size_t n, size_t per_cta,
-	uint32_t *__restrict__ parts, uint32_t *over) {
+radix_count16(const uint16_t *keys, size_t n, size_t per_cta,
+	uint32_t *parts, uint32_t *over) {
 	extern __shared__ __align__(16) uint32_t c16[];  // bin b: half b & 1 of word b >> 1
 	for (int i = threadIdx.x; i < kC16Bins / 8; i += kC16Threads)
 		reinterpret_cast<uint4 *>(c16)[i] = make_uint4(0, 0, 0, 0);
@@ -410,8 +410,8 @@ radix_count16(const uint16_t *__restrict__ keys, size_t n, size_t per_cta,
 // each bin's start within its block and the block's total.
 constexpr int kS16Bins = 512, kS16Blocks = kC16Bins / kS16Bins;
 __global__ void __launch_bounds__(1024)
-radix_sum16(const uint32_t *__restrict__ parts, uint32_t histograms,
-	const uint32_t *__restrict__ over, uint32_t *start, uint32_t *block_total) {
+radix_sum16(const uint32_t *parts, uint32_t histograms,
+	const uint32_t *over, uint32_t *start, uint32_t *block_total) {
 	constexpr int W = kS16Bins / 2;
 	__shared__ uint32_t s_lo[4][W], s_hi[4][W], s_warp[8];
 	const int x = threadIdx.x % W, y = threadIdx.x / W, lane = threadIdx.x & 31;
@@ -459,8 +459,8 @@ radix_sum16(const uint32_t *__restrict__ parts, uint32_t histograms,
 // bins of 1024 keys, its lanes between those for theirs.
 constexpr int kF16Threads = 512, kF16Window = 2048, kF16Chunk = 1024;
 __global__ void __launch_bounds__(kF16Threads)
-radix_fill16(uint16_t *out, size_t n, size_t per_cta, const uint32_t *__restrict__ start,
-	const uint32_t *__restrict__ block_total, bool in_place) {
+radix_fill16(uint16_t *out, size_t n, size_t per_cta, const uint32_t *start,
+	const uint32_t *block_total, bool in_place) {
 	__shared__ uint32_t s_block[kS16Blocks + 1], s_warp[4], s_win[kF16Window + 1];
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 	dev::pdl_wait();

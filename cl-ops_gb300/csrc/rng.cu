@@ -133,8 +133,8 @@ constexpr int kFillThreads = 256;
 // 4-byte stores, any count and alignment).
 template <int GEN, bool MAXINT, int V>
 __global__ void __launch_bounds__(kFillThreads)
-rng_fill_kernel(typename Gen<GEN>::S *__restrict__ states, size_t count,
-	uint32_t *__restrict__ out, size_t draws, uint32_t shift, uint32_t maxint) {
+rng_fill_kernel(typename Gen<GEN>::S *states, size_t count,
+	uint32_t *out, size_t draws, uint32_t shift, uint32_t maxint) {
 	using S = typename Gen<GEN>::S;
 	const size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
 	const size_t i0 = q * V;

@@ -50,10 +50,17 @@ constexpr int scan_min_blocks() {
 
 // One warp's block b of a tile, global -> padded shared memory.
 template <typename InT>
-__device__ __forceinline__ void load_block_scalar(const InT *__restrict__ in, size_t n,
-	size_t seg, InT *sin, int lane) {
-	for (int i = lane; i < kBlock; i += 32)
-		sin[pidx<InT>(i)] = (seg + i < n) ? in[seg + i] : (InT)0;
+__device__ __forceinline__ void load_block_scalar(const InT *in, size_t n, size_t seg, InT *sin,
+	int lane) {
+	constexpr int U = sizeof(InT) == 8 ? 4 : 8;  // loads in flight before their stores
+#pragma unroll 1
+	for (int i0 = lane; i0 < kBlock; i0 += 32 * U) {
+		InT v[U];
+#pragma unroll
+		for (int u = 0; u < U; ++u) v[u] = seg + i0 + 32 * u < n ? in[seg + i0 + 32 * u] : (InT)0;
+#pragma unroll
+		for (int u = 0; u < U; ++u) sin[pidx<InT>(i0 + 32 * u)] = v[u];
+	}
 }
 
 template <typename InT>
@@ -65,7 +72,7 @@ struct BlockRegs {
 
 // Issues the 16-byte loads of a warp's full blocks (prefetch).
 template <typename InT>
-__device__ __forceinline__ void issue_loads(BlockRegs<InT> &r, const InT *__restrict__ in,
+__device__ __forceinline__ void issue_loads(BlockRegs<InT> &r, const InT *in,
 	size_t wseg, int lane) {
 #pragma unroll
 	for (int b = 0; b < kBlocks; ++b) {

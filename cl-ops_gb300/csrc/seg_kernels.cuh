@@ -209,7 +209,7 @@ constexpr int kSegLookWindow = 8;     // predecessor statuses per round trip
 // of kSegLookWindow and a write-out with one base per digit.
 template <typename K, int KPT>
 __global__ void __launch_bounds__(kLThreads, 2)
-seg_pass(const K *__restrict__ kin, K *__restrict__ kout, SegPassArgs a) {
+seg_pass(const K *kin, K *kout, SegPassArgs a) {
 	constexpr int TILE = kLThreads * KPT;
 	constexpr int UKEYS = 16 * KPT;          // a unit's keys in one tile
 	constexpr int HALF = kLUnits / 2;        // 8 count rows

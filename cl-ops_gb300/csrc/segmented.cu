@@ -518,8 +518,8 @@ __global__ void __launch_bounds__(256) seg_heads(const uint64_t *off, uint32_t S
 // carry and does not look back.
 template <typename InT, typename OutT>
 __global__ void __launch_bounds__(scantile::kThreads, (scantile::scan_min_blocks<InT, OutT>()))
-seg_scan_lookback(const InT *__restrict__ in, OutT *__restrict__ out, uint64_t n,
-	const uint32_t *__restrict__ heads, const uint64_t *off, uint32_t S,
+seg_scan_lookback(const InT *in, OutT *out, uint64_t n,
+	const uint32_t *heads, const uint64_t *off, uint32_t S,
 	lb::TileStatus ts, int *dev_status, bool vec_ok) {
 	using namespace scantile;
 	using Acc = typename std::conditional<(sizeof(OutT) <= 4), uint32_t, uint64_t>::type;
@@ -548,8 +548,14 @@ seg_scan_lookback(const InT *__restrict__ in, OutT *__restrict__ out, uint64_t n
 	uint32_t tile = s_tile;
 	const uint64_t lo = s_lo, hi = s_hi;
 	if (tile >= num_tiles) return;
+	// The warp's 32 head words, one a lane.
+	auto head_word = [&](uint64_t seg) {
+		return seg + 32 * lane < n ? heads[(seg >> 5) + lane] : 0u;
+	};
+	uint32_t hw;
 	{
 		const uint64_t wseg = (uint64_t)tile * kTile + (uint64_t)warp * kWarpElems;
+		hw = head_word(wseg);
 		if (full_tile(tile)) {
 			BlockRegs<InT> r;
 			issue_loads<InT>(r, in, wseg, lane);
@@ -575,7 +581,8 @@ seg_scan_lookback(const InT *__restrict__ in, OutT *__restrict__ out, uint64_t n
 			const InT *sin = s_in + b * padded<InT>();
 			// 16 elements starting at a multiple of 16: one half of one word.
 			const uint64_t e0 = wseg + (uint64_t)b * kBlock + (uint64_t)lane * kItems;
-			hb[b] = e0 < n ? (heads[e0 >> 5] >> (uint32_t)(e0 & 31)) & 0xffffu : 0u;
+			const uint32_t w = __shfl_sync(0xffffffffu, hw, b * (kBlock / 32) + lane / 2);
+			hb[b] = e0 < n ? (w >> (16 * (lane & 1))) & 0xffffu : 0u;
 			Acc run = 0;
 #pragma unroll
 			for (int j = 0; j < kItems; ++j) {
@@ -625,7 +632,7 @@ seg_scan_lookback(const InT *__restrict__ in, OutT *__restrict__ out, uint64_t n
 		uint32_t nhw = 0;
 		if (next_full) {
 			issue_loads<InT>(r, in, nseg, lane);
-			nhw = heads[(nseg >> 5) + lane];
+			nhw = head_word(nseg);
 		}
 
 		// ---- tile status, lookback (warp 0) ------------------------------
@@ -746,6 +753,7 @@ seg_scan_lookback(const InT *__restrict__ in, OutT *__restrict__ out, uint64_t n
 		if (!have_next) break;
 
 		// ---- the next tile into shared memory ----------------------------
+		hw = next_full ? nhw : head_word(nseg);
 		if (next_full) {
 			store_loads<InT>(r, s_in, lane);
 		} else {
