@@ -627,7 +627,7 @@ __device__ __forceinline__ bool lookback_window(const uint32_t *status, int digi
 	return done;
 }
 
-// Lookback of sorts with few tiles (kGroupedTiles), which all run at about the
+// Lookback of sorts with few tiles (grouped_tiles), which all run at about the
 // same time: with windows a tile's prefix waits for its predecessors'
 // prefixes, a chain of tiles / 16 round trips. Here every tile also adds its
 // counts to its group's row (kGroup tiles; arrivals in the top bits), and a
@@ -1275,7 +1275,9 @@ struct TilesCfgPart {
 // about two waves (2^22 (u64, u32) pairs 305 against 323, (u32, u32) 143
 // against 159; 2^23 and 1100 tiles 610 against 576).
 template <int WORDS>
-constexpr size_t kGroupedTiles = WORDS == 1 ? 152 : 640;
+size_t grouped_tiles(CCLContext *ctx) {
+	return WORDS == 1 ? ctx->sm_count : ctx->sm_count * 21 / 5;
+}
 
 template <typename K, int PASSES>
 cudaError_t launch_upsweep_p(cudaStream_t s, const K *keys, size_t n, int base_shift,
@@ -1540,7 +1542,7 @@ cudaError_t sort_typed(const void *src, void *dst, void *vals, size_t n, int sor
 	if (fits(P2::kTile)) return go(P2(), Yes());
 	if (fits(P4::kTile)) return go(P4(), Yes());
 	if (fits(P6::kTile)) return go(P6(), Yes());
-	if (n <= Big::kTile * kGroupedTiles<Big::kWords>) return go(Big(), Yes());
+	if (n <= Big::kTile * grouped_tiles<Big::kWords>(ctx)) return go(Big(), Yes());
 	return loop_tiles<Big>(n, ctx) ? go(Big(), Loop()) : go(Big(), One());
 }
 

@@ -25,7 +25,7 @@ std::map<const void *, std::string> &names() {
 }
 std::vector<Launch> g_launches;
 std::map<const void *, void *> g_symbols;
-int g_device = 0;
+int g_device = 0, g_sms = 152;
 dim3 g_grid, g_block;
 size_t g_shared;
 cudaStream_t g_stream;
@@ -43,6 +43,7 @@ void fake_reset(int device) {
 	g_launches.clear();
 	g_device = device;
 }
+void fake_set_sms(int sms) { g_sms = sms; }
 int fake_launches(void) { return (int)g_launches.size(); }
 const char *fake_name(int i) { return g_launches[i].name.c_str(); }
 unsigned fake_grid(int i) { return g_launches[i].grid; }
@@ -108,7 +109,7 @@ cudaError_t cudaGetDevice(int *d) {
 	return cudaSuccess;
 }
 cudaError_t cudaDeviceGetAttribute(int *v, cudaDeviceAttr a, int) {
-	*v = a == cudaDevAttrMultiProcessorCount ? 152
+	*v = a == cudaDevAttrMultiProcessorCount ? g_sms
 		: a == cudaDevAttrComputeCapabilityMajor ? 10
 		: a == cudaDevAttrComputeCapabilityMinor ? 3
 		: a == cudaDevAttrMaxSharedMemoryPerBlockOptin ? 227 * 1024 : 1;

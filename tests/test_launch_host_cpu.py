@@ -105,3 +105,26 @@ def test_radix_sort_refusals(fake, n, src, dst, vb, bits, ok):
         fake.lib.clo_error_free(e)
     q.destroy()
     ctx.destroy()
+
+
+# Sorts of one tile an SM (one-word keys; 4.2 tiles with more) look back by
+# groups, whatever the number of SMs. (The last number in the kernel's name is
+# how it takes its tiles: 1 by groups.)
+@pytest.mark.parametrize("sms", [148, 152, 160])
+@pytest.mark.parametrize("values,tile,fifths", [(0, 15360, 5), (U32, 10240, 21)])
+def test_grouped_lookback_limit(fake, sms, values, tile, fifths):
+    fake.lib.fake_set_sms(sms)
+    ctx = fake.Context(0)
+    fake.lib.fake_set_sms(152)
+    q = fake.Queue(ctx)
+    s = fake.Sorter(ctx, "satradix", U32)
+    limit = sms * fifths // 5 * tile
+    a, b = fake.Buffer(ctx, 4 * limit + 4), fake.Buffer(ctx, 4 * limit + 4)
+    for n, grouped in ((limit, True), (limit + 1, False)):
+        names = _names(fake, (lambda: s.sort_kv_device(q, a, b, values, n)) if values else
+                       (lambda: s.sort_device(q, a, n, buf_out=b)))
+        passes = [x for x in names if "radix_pass_tiles" in x]
+        assert len(passes) == 4
+        assert all(("ELi1EEE" in x) == grouped for x in passes), (n, passes[0])
+    for x in (s, a, b, q, ctx):
+        x.destroy()
