@@ -17,8 +17,9 @@
 //   - bitonic_global_steps<g>: g consecutive steps with strides >= the
 //     tile, 2^g elements per thread held in registers;
 //   - bitonic_tile<.., finish>: the remaining steps T..1 of a stage.
-// A tile is the work of one CTA (2^K elements) or of a cluster of 2^LOGC
-// CTAs that exchange elements through distributed shared memory.
+// A tile is the work of one CTA (2^K elements). Sorts that one tile holds may
+// take a cluster of 2^LOGC CTAs, which exchange elements through distributed
+// shared memory.
 // The option settings that limit the grouping (maxps, maxsfs) take the
 // shared-memory rounds at the end of this file.
 // Sizes that are not a power of two are padded with the element type's
@@ -208,9 +209,9 @@ bitonic_global_steps_v(T *data, size_t groups, int stage, int step) {
 // With LOGC > 0 the tile spans a cluster, each CTA's shared memory holding
 // its 2^K consecutive elements. The phase on the cluster's bits takes the
 // layout L(T - RE), whose registers span the CTAs: it is entered by reading
-// the other CTAs' shared memory and left by writing into it (or entered
-// straight from global memory, in a finish). 2^15 4-byte elements sort in one
-// launch on 8 SMs in about a third of the time one SM takes for 2^14.
+// the other CTAs' shared memory and left by writing into it. 2^15 4-byte
+// elements sort in one launch on 8 SMs in 14.6 us, against 17 in five launches
+// of one-CTA tiles.
 //
 // No barrier is needed before a transpose's writes: a thread writes exactly
 // the slots it read itself in the transpose before (each slot has one owner
@@ -450,6 +451,7 @@ bitonic_tile(const T *src, T *dst, size_t n_src, size_t n_dst, int stage) {
 	constexpr int K = C::kK, LOGC = C::LOGC;
 	// Doubles travel as their bits (see ord).
 	constexpr bool kOrd = std::is_same<T, double>::value;
+	static_assert(LOGC == 0 || (SORT && !kOrd), "clusters sort up to 4-byte elements");
 	using U = typename std::conditional<kOrd, int64_t, T>::type;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	RegTile<U, C> t;
@@ -475,13 +477,8 @@ bitonic_tile(const T *src, T *dst, size_t n_src, size_t n_dst, int stage) {
 		}
 		tile_load(t, usrc + part, part < n_src ? n_src - part : 0, pad);
 	} else {
-		// The cluster phase reads its elements straight from global memory;
-		// the barrier's first half (the other CTAs have started, so their
-		// shared memory may be written) overlaps the loads.
-		if constexpr (LOGC > 0 && !kOrd) dev::cluster_arrive();
 #pragma unroll
 		for (int m = 0; m < C::R; ++m) t.r[m] = usrc[tile + (((size_t)m << C::LR) | t.g)];
-		if constexpr (LOGC > 0 && !kOrd) dev::cluster_wait();
 	}
 	auto work = [&](auto &w) {
 		if constexpr (SORT) {
@@ -499,20 +496,6 @@ bitonic_tile(const T *src, T *dst, size_t n_src, size_t n_dst, int stage) {
 #pragma unroll
 		for (int m = 0; m < C::R; ++m) special = special || ord_special(t.r[m]);
 		special = __syncthreads_or(special);
-		if constexpr (LOGC > 0) {
-			// One decision for the cluster. (A later barrier of the exchanges
-			// keeps the CTAs here until all have read: a cluster tile always
-			// has a cluster phase.)
-			__shared__ uint32_t s_special;
-			if (t.tid == 0) s_special = special;
-			dev::cluster_arrive();
-			dev::cluster_wait();
-			const uint32_t a = dev::smem_u32(&s_special);
-			uint32_t any = 0;
-#pragma unroll
-			for (int c = 0; c < C::kCluster; ++c) any |= dev::ld_dsmem<uint32_t>(dev::map_shared(a, c));
-			special = any != 0;
-		}
 		if (!special) {
 #pragma unroll
 			for (int m = 0; m < C::R; ++m) t.r[m] = ord(t.r[m]);
@@ -689,42 +672,48 @@ cudaError_t global_passes(T *d, size_t elems, int stage, int t, int maxg, double
 template <typename T>
 constexpr int kGlobalSteps = sizeof(T) == 4 ? 7 : sizeof(T) == 1 ? 5 : 6;
 
-// The sort with one tile configuration. `work` holds N elements (it may be
-// `dst` when n == N; null when one tile holds everything).
+// Stages 1 .. min(T, stages) of every tile of src's n elements into out, of
+// which n_out are written.
+template <typename T, typename C>
+cudaError_t launch_tile_sort(const T *src, T *out, size_t n, size_t n_out, size_t parts, int stages,
+	double bytes, const TimerNames &names, cudaStream_t s, unsigned &launches) {
+	auto kern = bitonic_tile<T, C, true>;
+	cudaError_t e = cudaSuccess;
+	if (C::kSmem > 48 * 1024)
+		e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::kSmem);
+	if (e != cudaSuccess) return e;
+	KernelTimer tm(names.tile_sort, s, bytes);
+	e = launch_chained(kern, (unsigned)parts, C::kThreads, C::kSmem, s, C::kCluster, src, out, n, n_out,
+		std::min(stages, C::TL));
+	tm.stop();
+	launches++;
+	return e;
+}
+
+// The sort with one-CTA tiles. `work` holds N elements (it is `dst` when
+// n == N or one tile holds everything).
 template <typename T, typename C>
 cudaError_t run_tiles(const T *src, T *dst, T *work, size_t n, int logN,
 	const TimerNames &names, cudaStream_t s, unsigned &launches) {
 	constexpr int K = C::kK;
 	const size_t N = (size_t)1 << logN;
-	const int TL = C::TL;
-	auto sort_k = bitonic_tile<T, C, true>;
+	const double pass_bytes = 2.0 * (double)N * sizeof(T);
+	if (logN <= K)
+		return launch_tile_sort<T, C>(src, dst, n, n, 1, logN, pass_bytes, names, s, launches);
 	auto fin_k = bitonic_tile<T, C, false>;
 	cudaError_t e = cudaSuccess;
-	if (C::kSmem > 48 * 1024) {
-		e = cudaFuncSetAttribute(sort_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::kSmem);
-		if (e == cudaSuccess)
-			e = cudaFuncSetAttribute(fin_k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-				(int)C::kSmem);
-		if (e != cudaSuccess) return e;
-	}
-	const bool one = logN <= TL;
-	const size_t parts = one ? (size_t)C::kCluster : N >> K;
-	const double pass_bytes = 2.0 * (double)N * sizeof(T);
-	{
-		KernelTimer tm(names.tile_sort, s, pass_bytes);
-		e = launch_chained(sort_k, (unsigned)parts, C::kThreads, C::kSmem, s, C::kCluster, src,
-			one ? dst : work, n, one ? n : N, std::min(logN, TL));
-		tm.stop();
-		launches++;
-	}
-	for (int stage = TL + 1; stage <= logN && e == cudaSuccess; ++stage) {
+	if (C::kSmem > 48 * 1024)
+		e = cudaFuncSetAttribute(fin_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::kSmem);
+	if (e == cudaSuccess)
+		e = launch_tile_sort<T, C>(src, work, n, N, N >> K, logN, pass_bytes, names, s, launches);
+	for (int stage = K + 1; stage <= logN && e == cudaSuccess; ++stage) {
 		// A stage leaves blocks of padding alone as they are.
 		const size_t elems = ((n + ((size_t)1 << stage) - 1) >> stage) << stage;
-		e = global_passes<T>(work, elems, stage, TL, kGlobalSteps<T>, pass_bytes, names, s, launches);
+		e = global_passes<T>(work, elems, stage, K, kGlobalSteps<T>, pass_bytes, names, s, launches);
 		if (e != cudaSuccess) break;
 		const bool last = stage == logN;
 		KernelTimer tf(names.tile_finish, s, pass_bytes);
-		e = launch_chained(fin_k, (unsigned)(elems >> K), C::kThreads, C::kSmem, s, C::kCluster,
+		e = launch_chained(fin_k, (unsigned)(elems >> K), C::kThreads, C::kSmem, s, 1,
 			(const T *)work, last ? dst : work, N, last ? n : N, stage);
 		tf.stop();
 		launches++;
@@ -818,7 +807,8 @@ cudaError_t sort_typed(const T *src, T *dst, size_t n, int max_ps, int max_sfs,
 			e = cudaMemcpyAsync(dst, tmp, n * sizeof(T), cudaMemcpyDeviceToDevice, s);
 	} else if (logN > SmallTile<T>::kK && logN <= kOneTile<T>) {
 		if constexpr (sizeof(T) <= 4)
-			e = run_tiles<T, ClusterTile<T>>(src, dst, work, n, logN, names, s, launches);
+			e = launch_tile_sort<T, ClusterTile<T>>(src, dst, n, n, ClusterTile<T>::kCluster, logN,
+				2.0 * (double)N * sizeof(T), names, s, launches);
 	} else {
 		bool big = false;
 		if constexpr (sizeof(T) == 8) {
