@@ -81,19 +81,23 @@ using If = typename std::conditional<C, A, B>::type;
 // Threads, tile and resident CTAs per SM (registers: 65536 / (CTAs x
 // threads)), and whether the current tile waits in shared memory while the
 // next one is loaded (KEEP: each thread parks its own vectors, conflict-free;
-// the two tiles' registers otherwise leave one CTA fewer an SM, or spills).
+// two tiles' registers leave one CTA fewer an SM or spill more).
 // The tile rate is bounded by the lookback (a window of 64 tiles a round trip,
 // about 80 tiles a microsecond), so narrow types take tiles twice as long.
-// Measured at 2^28 (us): uint -> ulong two CTAs 559, three with KEEP 519, four
+// Measured at 2^28 (us): uint -> ulong two CTAs 559, three with KEEP 517, four
 // 547; ulong -> ulong 804 / 694 (two CTAs) / 1023 (three); uint -> uint
 // 16384-element tiles 380 / 356 (two) / 498 (three), 8192 406; uchar -> uint
-// 16384 255 (three), 8192 404. Windows of 96 and 128 tiles
-// and 512-thread CTAs were slower.
+// 16384 256 (three) / 275 (two), 8192 404; ushort -> uint 310 (three, with 168
+// bytes of spills a thread) / 293 (two, none), 2^24 30.5 / 24.4. Spills that
+// remain, a thread: uchar -> uint 84 bytes, ulong -> ulong 60, uint -> uint
+// 48, uint -> ulong in 4096-element tiles 20. Windows of 96 and 128 tiles and
+// 512-thread CTAs were slower.
 template <typename InT, typename OutT>
 using ScanBig = If<kOneShape<InT, OutT>, ScanCfg<InT, OutT, 256, 8192, 1>,
 	If<sizeof(OutT) == 8, If<sizeof(InT) == 8, ScanCfg<InT, OutT, 256, 8192, 2, true>,
 		If<sizeof(InT) == 4, ScanCfg<InT, OutT, 256, 8192, 3, true>, ScanCfg<InT, OutT, 256, 8192, 2>>>,
-	If<sizeof(InT) == 4, ScanCfg<InT, OutT, 256, 16384, 2, true>, ScanCfg<InT, OutT, 256, 16384, 3>>>>;
+	If<sizeof(InT) == 4, ScanCfg<InT, OutT, 256, 16384, 2, true>,
+		ScanCfg<InT, OutT, 256, 16384, sizeof(InT) == 2 ? 2 : 3>>>>;
 // From kSmallMax to kMidMax elements uint -> ulong tiles stay in registers: with
 // about one tile a CTA nothing is prefetched (2^22 16.2 us against 17.9).
 constexpr size_t kMidMax = (size_t)1 << 23;
