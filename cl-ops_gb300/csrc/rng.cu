@@ -173,13 +173,19 @@ cudaError_t launch_fill(void *states, size_t count, uint32_t *out, size_t draws,
 
 // Counts from which a thread takes four states (whole rows of 16-byte stores
 // need count % 4 == 0 and an aligned output too); below, one state a thread
-// fills the SMs better. us, four / one: mwc64x 65536 x 64 5.8 / 4.0, 262144 x
-// 32 6.6 / 6.2, 2^20 x 32 21.4 / 19.5, 2^22 x 32 88.2 / 90.3; parkmiller
-// 262144 x 32 6.6 / 6.8, 2^20 x 32 20.1 / 22.8. Counts that are no multiple of
-// four (2^22 - 1 mwc64x x 32): 138 us, whose rows' stores meet the 32-byte
-// sectors unaligned; 524 with four states a thread one after the other.
+// keeps the SMs fuller. us, four / one, states x draws: mwc64x 65536 x 64 5.8 /
+// 4.0, 2^20 x 32 20.9 / 19.5, 2^22 x 8 26.4 / 23.6, 2^22 x 64 157 / 157, 2^23 x
+// 32 174 / 179 (lcg and xorshift64 alike); 16-byte states: xorshift128 2^20 x
+// 32 22.8 / 19.5, 2^21 x 8 18.2 / 13.4, 2^22 x 8 34.1 / 32.0, 2^22 x 32 92.6 /
+// 96.5, tauslcg 2^21 x 8 18.2 / 14.9, x 32 42.7 / 47.0; parkmiller 262144 x 32
+// 6.6 / 6.8, 2^20 x 32 20.1 / 22.8, 2^22 x 8 20.6 / 26.3. Counts that are no
+// multiple of four (2^22 - 1 mwc64x x 32): 138 us, whose rows' stores meet the
+// 32-byte sectors unaligned; 524 with four states a thread one after the other.
 template <int GEN>
-constexpr size_t kVecMin = GEN == RNG_PARKMILLER ? (size_t)1 << 18 : (size_t)1 << 21;
+size_t vec_min(size_t draws) {
+	if (GEN == RNG_PARKMILLER) return (size_t)1 << 18;
+	return sizeof(typename Gen<GEN>::S) == 16 && draws >= 32 ? (size_t)1 << 21 : (size_t)1 << 23;
+}
 
 template <int GEN>
 cudaError_t fill_gen(void *states, size_t count, uint32_t *out, size_t draws,
@@ -187,7 +193,7 @@ cudaError_t fill_gen(void *states, size_t count, uint32_t *out, size_t draws,
 	using S = typename Gen<GEN>::S;
 	const uint32_t shift = 32u - bits;
 	const bool vec = (count % 4) == 0 && ((uintptr_t)out % 16) == 0 &&
-		count >= kVecMin<GEN>;
+		count >= vec_min<GEN>(draws);
 	KernelTimer t("rng_fill", s, (double)count * (4.0 * draws + 2.0 * sizeof(S)));
 	const cudaError_t e = maxint
 		? (vec ? launch_fill<GEN, true, 4>(states, count, out, draws, shift, maxint, s)
