@@ -764,8 +764,11 @@ cudaError_t run_rounds(T *d, int logN, int max_ps, int max_sfs,
 //   32 elements a thread: 2^16 22.7 / 27.3 / 41, 2^24 657 / 632 / 659; clusters
 //   of eight over 2^12: 2^16 26, 2^20 63, 2^24 755; 2^15 14.6 in one cluster
 //   against 17 in five launches.
-//   double, 2^11 by 8 / 2^13 by 16: 2^16 36 / 63, 2^20 138 / 132, 2^22 496 /
-//   500, 2^24 2358 / 2141; clusters of eight over 2^12 by 16: 2^16 44.
+//   double, 2^11 by 8 / 2^13 by 16: 2^16 37 / 63, 2^19 86 / 110, 2^20 138 / 132,
+//   1.5 x 10^6 206 / 236, 2^22 496 / 499, 5 x 10^6 746 / 721, 2^24 2357 / 2145
+//   (the compares bound the large sorts); clusters of eight over 2^12 by 16:
+//   2^16 44. long: 2^20 102 / 105, 2^22 346 / 392, 5 x 10^6 488 / 560, 2^23 680
+//   / 729, 2^24 1789 / 1797, 2^25 3833 / 3771.
 //   char, 32 / 16 elements a thread: 2^16 27 / 26, 2^24 673 / 729.
 template <typename T>
 using SmallTile = typename std::conditional<sizeof(T) == 8, TileCfg<T, 11, 0, 3>,
@@ -774,7 +777,9 @@ template <typename T>
 using ClusterTile = TileCfg<T, 12, 3, sizeof(T) == 1 ? 5 : 4>;
 template <typename T>
 constexpr int kOneTile = sizeof(T) == 8 ? 11 : 15;
-constexpr int kBigDoubleMin = 23;  // log2: 8-byte tiles of 2^13 from here
+// log2 of the padded size from which 8-byte elements take tiles of 2^13.
+template <typename T>
+constexpr int kBigTileMin = std::is_same<T, double>::value ? 23 : 25;
 
 template <typename T>
 cudaError_t sort_typed(const T *src, T *dst, size_t n, int max_ps, int max_sfs,
@@ -812,7 +817,7 @@ cudaError_t sort_typed(const T *src, T *dst, size_t n, int max_ps, int max_sfs,
 	} else {
 		bool big = false;
 		if constexpr (sizeof(T) == 8) {
-			big = logN >= kBigDoubleMin;
+			big = logN >= kBigTileMin<T>;
 			if (big) e = run_tiles<T, TileCfg<T, 13, 0, 4>>(src, dst, work, n, logN, names, s, launches);
 		}
 		if (!big) e = run_tiles<T, SmallTile<T>>(src, dst, work, n, logN, names, s, launches);

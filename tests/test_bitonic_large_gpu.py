@@ -1,6 +1,7 @@
 """The bitonic sorters' other tiles, against the network replay (bit for bit):
-8-byte elements beyond 2^22, which take tiles of 2^13 (whole tiles of padding
-at 2^22 + 1), with and without values whose order is not total; the limit of
+8-byte elements at the sizes that take tiles of 2^13 (doubles beyond 2^22,
+with and without values whose order is not total, integers beyond 2^24; whole
+tiles of padding one element past them); the limit of
 the one-launch cluster (2^15); sbitonic at the sizes of the global passes."""
 import numpy as np
 import pytest
@@ -27,6 +28,12 @@ def test_eight_byte_large_tiles(clops, ctx, queue, code, dt, special, n, offset)
     elif special == "one_tile":
         a[70000:75000] = _specials(a[70000:75000].copy())
     _check(clops, ctx, queue, "abitonic", code, a, offset=offset)
+
+
+@pytest.mark.parametrize("code,dt", [(6, np.int64), (7, np.uint64)])
+@pytest.mark.parametrize("n", [1 << 24, (1 << 24) + 1])
+def test_integers_at_the_line(clops, ctx, queue, code, dt, n):
+    _check(clops, ctx, queue, "abitonic", code, keys_of_type(907, n, dt), offset=n & 1)
 
 
 @pytest.mark.parametrize("code,dt", [(10, np.float64), (6, np.int64)])
