@@ -12,9 +12,10 @@
 //   2. radix_upsweep_w reads the keys once, builds the 256-bin histogram of every digit position, and
 //      its last CTA scans them into digit bases and writes the plan: which
 //      passes run and between which buffers;
-//   3. per digit position, radix_pass_tiles (one launch per pass), one CTA
-//      per tile (15360 32-bit keys; 7168 pairs of a 64-bit key and a
-//      32-bit value), tiles claimed in order from a counter:
+//   3. per digit position, radix_pass_tiles (one launch per pass), a CTA for
+//      each tile or, in large sorts, resident CTAs that take tile after tile
+//      (15360 32-bit keys; 7168 pairs of a 64-bit key and a 32-bit value),
+//      tiles claimed in order from a counter:
 //      a. keys are loaded in half-warp units (a unit's keys are in index
 //         order; full tiles of 32-bit keys arrive by bulk copy into shared
 //         memory), the tile's digit counts are published for the decoupled
@@ -1230,7 +1231,8 @@ radix_cluster(const K *kin, K *kout, const V *vin, V *vout, uint32_t n, uint32_t
 // takes: keys per thread and resident CTAs per SM, each the measured best
 // at 2^27 - 2^28 elements (larger tiles spread the per-tile work -- row
 // clears and scans, the lookback -- over more keys; the limits are 128
-// registers a thread without spills and two CTAs' shared memory per SM).
+// registers a thread, without spills but for the 12 to 16 bytes of (u32, u64)
+// pairs, and two CTAs' shared memory per SM).
 // 32-bit keys: 15360-key tiles; 64-bit keys or 32-bit pairs: 10240;
 // 12-byte pairs (bulk-loaded): 7168, 5120 for those loaded lane by lane
 // (8- and 16-bit keys with 64-bit values); 16-byte pairs 5120.
@@ -1325,9 +1327,13 @@ cudaError_t launch_upsweep(int passes, cudaStream_t s, const K *keys, size_t n,
 // Passes of at least three waves of tiles run as resident CTAs that take tile
 // after tile: no gaps between CTAs, and a pass that the plan skips costs one
 // wave of empty CTAs instead of one per tile (2^28 equal keys 353 -> 178 us a
-// sort). Below, one CTA a tile is faster (u32 keys, us, one / loop: 5 x 10^6
-// 113 / 127, 10^7 192 / 192, 1.4 x 10^7 230 / 226; u64 4 x 10^6 228 / 239, 5 x 10^7
-// 1850 / 1771; (u64, u32) 5 x 10^6 390 / 401, 2^25 1843 / 1807).
+// sort). Below, one CTA a tile is faster. us, one / loop: u32 keys 5 x 10^6
+// 113 / 127, 10^7 193 / 192, 1.4 x 10^7 231 / 225, 2^27 1682 / 1622; u64 keys 4 x
+// 10^6 228 / 239, 10^7 458 / 453, 2^27 4721 / 4597; (u32, u32) 10^7 286 / 295, 2 x
+// 10^7 505 / 498, 2^27 2781 / 2796; (u64, u32) 7 x 10^6 488 / 498, 1.4 x 10^7
+// 872 / 857, 2^27 6835 / 6856; (u64, u64) 10^7 796 / 781, 2^27 8692 / 8675. Pairs
+// of 3 to 5 waves lose up to 3% and (u32, u64) 1 to 3% throughout (2 x 10^7 636 /
+// 651, 2^27 3658 / 3723); they loop all the same, for the passes that are skipped.
 constexpr size_t kLoopWaves = 3;
 template <typename TC>
 bool loop_tiles(size_t n, CCLContext *ctx) {

@@ -36,7 +36,8 @@ __device__ __forceinline__ uint32_t digit_of(K k, int shift) {
 //   class A CTA layout    (threads, keys per thread): 128 x 8, 256 x 8
 //   class B CTA layout    512 x 16, 256 x 16, 1024 x 16
 //   long-segment pass     keys per thread of 256-thread tiles: 56, 48, 40
-//                         (8-byte keys: 32, 28, 24)
+//                         (8-byte keys: 32, 28, 24); small buffers take 14
+//                         (8) whatever the shape (kSmallLong)
 //   CTA classes' digits   8 or 4 bits per local LSD pass
 // Keys of 8 bytes halve the CTA classes' keys per thread. The class
 // boundaries follow from the layouts: a segment goes to the warp class up
@@ -71,10 +72,15 @@ constexpr int long_kpt(int idx) {
 	return sizeof(K) <= 4 ? (idx == 0 ? 56 : idx == 1 ? 48 : idx == 2 ? 40 : 14)
 						  : (idx == 0 ? 32 : idx == 1 ? 28 : idx == 2 ? 24 : 8);
 }
-// Buffers that would not give every SM a tile of the shape's size take a
-// quarter of it (kSmallLong), whatever the shape: a 14336-key tile alone on
-// its SM takes 18 us a pass (100,000 keys in 100 segments, some of them long:
-// 95.6 us a sort, 58.7 with the small tiles).
+// Buffers that would not give every SM a tile of the shape's size (2.2 x 10^6
+// keys of up to 32 bits, 1.2 x 10^6 of 64 on 152 SMs) take a quarter of it
+// (kSmallLong), whatever the shape: a 14336-key tile alone on its SM takes 18 us
+// a pass. us a sort of 16 / 200 segments of log-normal length (sigma 2), the
+// shape's tiles against the small ones: 32-bit keys 3 x 10^5 83 : 62 / 98 : 59,
+// 1.2 x 10^6 99 : 88 / 116 : 77, 1.6 x 10^6 102 : 103 / 117 : 91, 2.1 x 10^6 107 :
+// 119 / 123 : 97, 3.5 x 10^6 122 : 160 / 123 : 130; 64-bit keys 6 x 10^5 120 :
+// 120 / 148 : 101, 1.2 x 10^6 142 : 174 / 158 : 138, 2.1 x 10^6 172 : 251 / 165 :
+// 198. Few long segments would change sooner, many later; the line lies between.
 constexpr int kSmallLong = 3;
 template <typename K>
 constexpr uint32_t long_tile(int idx) {
