@@ -2,7 +2,8 @@
 // at (staged_scan in scan.cu): tiles of 8192 elements staged in shared memory
 // (scan_tile.cuh), read and written in whole lines whatever the types and the
 // alignment; a lane scans 16 consecutive elements there. Bound by the shared
-// memory's wavefronts (uint -> uchar 2^28: 322 us, 61% of the copy rate).
+// memory's pipe, 70% busy, and the barriers around the lookback (uint -> uchar
+// 2^28: 322 us, 61% of the copy rate).
 #pragma once
 
 #include <stddef.h>
